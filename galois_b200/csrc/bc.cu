@@ -17,13 +17,20 @@
 //  * batch 2..64 (multi-source, cf. MRBC's source batching in
 //    lonestar/analytics/distributed/betweennesscentrality/bc_mr.cpp:84-158):
 //    per vertex and level a 64-bit mask of the sources that reach it at that
-//    level; sigma (fp64) and dep (fp32) stored vertex-major [n][64] so lane s
+//    level; path counts (fp64) stored vertex-major [n][64] so lane s
 //    of a warp owns source s and s+32 and a row is one coalesced load.
-//    Forward levels pull: a vertex still missing sources scans its neighbours
-//    32 at a time, a ballot keeps the neighbours in the frontier for a needed
-//    source, and only those rows of sigma are read.  Backward levels walk the
-//    stored masks.  Light vertices are owned by one warp (no atomics); heavy
-//    vertices are split into tiles that combine with atomics.
+//    Levels pull, 32 consecutive vertices per warp task: the arcs of the
+//    task's vertices are walked together, 32 * kMsU column and mask loads in
+//    flight, and the arcs whose neighbour carries a needed source are taken
+//    four at a time (eight row loads in flight per lane), whichever vertices
+//    they belong to.  A vertex's row holds sigma until its backward level and
+//    (1 + dep) / sigma from then on, the one value its predecessors add: one
+//    8-byte load per (arc, source) and no division per arc.  Light vertices
+//    are owned by one warp (no atomics); heavy vertices are split into tiles
+//    that combine with atomics.  64 sources of RMAT-20 (31 M arcs, degree
+//    order): one vertex per warp with one row in flight and (1 + dep) / sigma
+//    divided per arc took 19.7 ms (20 % issue-active, stalled on barriers and
+//    on one load after another); this takes 8.4 ms.
 //  bc accumulates in fp64 across sources and batches; the output is fp32.
 
 #include "device_common.cuh"
@@ -47,8 +54,7 @@ struct BcCtl {
   uint32_t levels;
   uint32_t any[4];  // per-level "something reached" flags (ring)
   uint32_t level_needed;
-  uint32_t pad;
-  unsigned long long scanned;
+  uint32_t next[4];  // batched kernel: next task of a pass (ring over the passes)
 };
 
 // ---------------------------------------------------------------- batched --
@@ -63,8 +69,7 @@ struct MsArgs {
   unsigned long long* lm;  // [lcap][n] level masks
   uint32_t lcap;
   unsigned long long* visit;  // [n]
-  double* sigma;              // [n][64]
-  float* dep;                 // [n][64]
+  double* rows;               // [n][64] sigma, then (1 + dep) / sigma (see the file comment)
   double* bc;                 // [n]
   double* hacc;               // [2][nheavy][64] backward partial sums of heavy vertices; level L adds
                               // into half L & 1 and zeroes the other half (a store to a word this
@@ -75,19 +80,23 @@ struct MsArgs {
   BcCtl* ctl;
 };
 
+constexpr int kMsBlock = 256;
+constexpr int kMsU = 4;  // 32-arc steps of column and mask loads in flight
+
 __device__ __forceinline__ unsigned long long shfl64(unsigned long long x, int k) {
   return __shfl_sync(kFull, x, k);
 }
 
+// What a batch reads before writing it: the masks of level 0, the visited
+// masks, and the rows (atomically added to), level-1 masks and backward sums
+// of the heavy vertices.  Every other word is written before it is read.
 __global__ void ms_init(MsArgs a) {
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = tid; i < (uint64_t)a.n * 64; i += stride) {
-    a.sigma[i] = 0.0;
-    a.dep[i] = 0.f;
-  }
-  for (uint64_t i = tid; i < (uint64_t)a.lcap * a.n; i += stride) a.lm[i] = 0ull;
-  for (uint64_t v = tid; v < a.n; v += stride) a.visit[v] = 0ull;
+  for (uint64_t v = tid; v < a.n; v += stride) a.lm[v] = a.visit[v] = 0ull;
+  for (uint64_t i = tid; i < (uint64_t)a.fs.nheavy * 64; i += stride)
+    a.rows[(uint64_t)a.fs.heavy_list[i >> 6] * 64 + (i & 63)] = 0.0;
+  for (uint64_t i = tid; i < a.fs.nheavy; i += stride) a.lm[(uint64_t)a.n + a.fs.heavy_list[i]] = 0ull;
   for (uint64_t i = tid; i < 2ull * a.bs.nheavy * 64; i += stride) a.hacc[i] = 0.0;
   for (uint64_t i = tid; i < a.bs.nheavy; i += stride) a.hidx[a.bs.heavy_list[i]] = (uint32_t)i;
 }
@@ -99,95 +108,136 @@ __global__ void ms_seed(MsArgs a) {
       const uint32_t s = a.srcs[b];
       a.lm[s] |= 1ull << b;
       a.visit[s] |= 1ull << b;
-      a.sigma[(uint64_t)s * 64 + b] = 1.0;
+      a.rows[(uint64_t)s * 64 + b] = 1.0;
     }
   }
 }
 
-// Forward work for one (vertex, arc range) by a whole warp.  Returns the
-// newly reached source mask; sA/sB receive the sigma sums for sources lane
-// and lane+32.
-__device__ __forceinline__ unsigned long long ms_forward_range(const MsArgs& a, const unsigned long long* cur,
-                                                               unsigned long long need, uint64_t b, uint64_t e,
-                                                               double& sA, double& sB) {
+// Takes the arcs of one 32-arc step that carry a needed source (f != 0), four
+// at a time so that eight row loads are in flight per lane: begin(owner) once
+// per arc in arc order (all lanes; the owner is warp-uniform), then add(xA, xB)
+// with the neighbour's values for sources lane and lane + 32 (0 where the mask
+// has no bit) and the arc's mask.
+template <class Begin, class Add>
+__device__ __forceinline__ void ms_take(const double* rows, uint32_t owner, uint32_t v, unsigned long long f,
+                                        Begin&& begin, Add&& add) {
+  const uint32_t lane = lane_id();
+  unsigned hits = __ballot_sync(kFull, f != 0);
+  while (hits) {
+    double xA[4], xB[4];
+    unsigned long long fk[4];
+    uint32_t own[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool on = hits != 0;
+      const int k = on ? __ffs(hits) - 1 : 0;
+      hits &= hits - 1;
+      own[j] = __shfl_sync(kFull, owner, k);
+      const double* row = rows + (uint64_t)__shfl_sync(kFull, v, k) * 64;
+      const unsigned long long m = shfl64(f, k);
+      fk[j] = on ? m : 0ull;
+      xA[j] = ((fk[j] >> lane) & 1ull) ? row[lane] : 0.0;
+      xB[j] = ((fk[j] >> (lane + 32)) & 1ull) ? row[lane + 32] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (fk[j] == 0) break;
+      begin(own[j]);
+      add(xA[j], xB[j], fk[j]);
+    }
+  }
+}
+
+// Sums over one arc range of one vertex, by a whole warp: the rows of the
+// neighbours whose mask shares a source with `need`; returns the sources seen.
+__device__ __forceinline__ unsigned long long ms_range(const double* rows, const uint32_t* col,
+                                                       const unsigned long long* masks, unsigned long long need,
+                                                       uint64_t b, uint64_t e, double& sA, double& sB) {
   const uint32_t lane = lane_id();
   unsigned long long acc = 0;
-  for (uint64_t base = b; base < e; base += 32) {
-    const uint64_t j = base + lane;
-    uint32_t v = 0;
-    unsigned long long f = 0;
-    if (j < e) {
-      v = ldg(a.in_col + j);
-      f = cur[v] & need;
+  for (uint64_t base = b; base < e; base += 32 * kMsU) {
+    uint32_t v[kMsU];
+    unsigned long long f[kMsU];
+#pragma unroll
+    for (int k = 0; k < kMsU; ++k) {
+      const uint64_t j = base + 32 * k + lane;
+      v[k] = j < e ? ldg(col + j) : 0xFFFFFFFFu;
     }
-    unsigned hits = __ballot_sync(kFull, f != 0);
-    while (hits) {
-      const int k = __ffs(hits) - 1;
-      hits &= hits - 1;
-      const uint32_t vk = __shfl_sync(kFull, v, k);
-      const unsigned long long fk = shfl64(f, k);
-      acc |= fk;
-      const double* row = a.sigma + (uint64_t)vk * 64;
-      if ((fk >> lane) & 1ull) sA += row[lane];
-      if ((fk >> (lane + 32)) & 1ull) sB += row[lane + 32];
-    }
+#pragma unroll
+    for (int k = 0; k < kMsU; ++k) f[k] = v[k] != 0xFFFFFFFFu ? masks[v[k]] & need : 0ull;
+#pragma unroll
+    for (int k = 0; k < kMsU; ++k)
+      ms_take(rows, 0u, v[k], f[k], [](uint32_t) {}, [&](double xA, double xB, unsigned long long m) {
+        acc |= m;
+        sA += xA;
+        sB += xB;
+      });
   }
   return acc;
 }
 
-// Backward work for one (vertex, arc range): sums (1+dep[w])/sigma[w] over
-// successors w for the sources in cv.
-__device__ __forceinline__ void ms_backward_range(const MsArgs& a, const unsigned long long* nextl,
-                                                  unsigned long long cv, uint64_t b, uint64_t e, double& dA,
-                                                  double& dB) {
-  const uint32_t lane = lane_id();
-  for (uint64_t base = b; base < e; base += 32) {
-    const uint64_t j = base + lane;
-    uint32_t w = 0;
-    unsigned long long g = 0;
-    if (j < e) {
-      w = ldg(a.col + j);
-      g = nextl[w] & cv;
-    }
-    unsigned hits = __ballot_sync(kFull, g != 0);
-    while (hits) {
-      const int k = __ffs(hits) - 1;
-      hits &= hits - 1;
-      const uint32_t wk = __shfl_sync(kFull, w, k);
-      const unsigned long long gk = shfl64(g, k);
-      const uint64_t r = (uint64_t)wk * 64;
-      if ((gk >> lane) & 1ull) dA += (1.0 + (double)a.dep[r + lane]) / a.sigma[r + lane];
-      if ((gk >> (lane + 32)) & 1ull) dB += (1.0 + (double)a.dep[r + lane + 32]) / a.sigma[r + lane + 32];
-    }
-  }
+// The same sums for the 32 vertices of a chunk, whose lanes supply (first arc,
+// arc count, needed sources).  done(owner lane, sources seen, sA, sB) is called
+// by all lanes once per vertex that has an arc with a needed source.
+template <class Done>
+__device__ __forceinline__ void ms_chunk(const double* rows, const uint32_t* col, const unsigned long long* masks,
+                                         unsigned long long need, uint64_t b, uint32_t d, Done&& done) {
+  uint32_t cur = 32;  // no owner yet
+  unsigned long long acc = 0;
+  double sA = 0.0, sB = 0.0;
+  warp_expand_mlp<kMsU, unsigned long long>(
+      b, d, 0u, [&](bool valid, uint64_t e, uint32_t) { return valid ? ldg(col + e) : 0u; },
+      [&](bool valid, uint64_t, uint32_t v, uint32_t) { return valid ? masks[v] : 0ull; },
+      [&](bool, uint32_t owner, uint32_t, uint32_t v, unsigned long long f) {
+        f &= shfl64(need, owner);
+        ms_take(
+            rows, owner, v, f,
+            [&](uint32_t o) {
+              if (o == cur) return;
+              if (cur < 32) done(cur, acc, sA, sB);
+              cur = o;
+              acc = 0;
+              sA = sB = 0.0;
+            },
+            [&](double xA, double xB, unsigned long long m) {
+              acc |= m;
+              sA += xA;
+              sB += xB;
+            });
+      });
+  if (cur < 32) done(cur, acc, sA, sB);
 }
 
-// Lanes filter 32 consecutive vertices; the warp then serves the selected
-// ones one by one.  fn(v) is called by the whole warp.
+// The tasks of one pass, handed out in order (heavy tiles, then chunks: on a
+// degree-ordered graph the longest first), the next one asked for before the
+// current one runs.
 template <class Fn>
-__device__ __forceinline__ void ms_for_light(const MsArgs& a, const SweepSched& s, const uint64_t* offs,
-                                             uint64_t gwarp, uint64_t nwarps, Fn&& select_and_run) {
+__device__ __forceinline__ void ms_tasks(uint32_t* next, uint64_t total, Fn&& fn) {
   const uint32_t lane = lane_id();
-  const uint64_t nchunks = ((uint64_t)a.n + 31) >> 5;
-  for (uint64_t c = gwarp; c < nchunks; c += nwarps) {
-    const uint64_t v = (c << 5) + lane;
-    bool light = false;
-    if (v < a.n) light = ldg(offs + v + 1) - ldg(offs + v) <= s.heavy;
-    select_and_run((uint32_t)v, v < a.n && light);
+  uint32_t t = 0;
+  if (lane == 0) t = atomicAdd(next, 1u);
+  t = __shfl_sync(kFull, t, 0);
+  while (t < total) {
+    uint32_t t2 = 0;
+    if (lane == 0) t2 = atomicAdd(next, 1u);
+    fn(t);
+    t = __shfl_sync(kFull, t2, 0);
   }
 }
 
-__global__ void __launch_bounds__(kBcBlock) ms_persistent(MsArgs a) {
+__global__ void __launch_bounds__(kMsBlock, 4) ms_persistent(MsArgs a) {
   BcCtl* ctl = a.ctl;
   const uint64_t deadline = kernel_deadline();
-  const uint64_t gtid = blockIdx.x * (uint64_t)kBcBlock + threadIdx.x;
-  const uint64_t gthreads = (uint64_t)gridDim.x * kBcBlock;
+  const uint64_t gtid = blockIdx.x * (uint64_t)kMsBlock + threadIdx.x;
+  const uint64_t gthreads = (uint64_t)gridDim.x * kMsBlock;
   const uint64_t gwarp = gtid >> 5, nwarps = gthreads >> 5;
   const uint32_t lane = lane_id();
   const unsigned long long active = a.nsrc >= 64 ? ~0ull : ((1ull << a.nsrc) - 1ull);
+  const uint32_t nchunks = (uint32_t)(((uint64_t)a.n + 31) >> 5);
+  uint32_t pass = 0;
   // ---- forward: level masks and path counts ----------------------------------
   uint32_t L = 0;
-  for (;; ++L) {
+  for (;; ++L, ++pass) {
     if (L + 1 >= a.lcap) {
       if (gtid == 0) {
         ctl->level_needed = L + 2;
@@ -197,104 +247,152 @@ __global__ void __launch_bounds__(kBcBlock) ms_persistent(MsArgs a) {
     }
     const unsigned long long* cur = a.lm + (uint64_t)L * a.n;
     unsigned long long* nxt = a.lm + (uint64_t)(L + 1) * a.n;
-    if (gtid == 0) ctl->any[(L + 2) & 3] = 0;
-    ms_for_light(a, a.fs, a.in_offs, gwarp, nwarps, [&](uint32_t v, bool light) {
-      const unsigned long long need = light ? (~a.visit[v] & active) : 0ull;
-      unsigned sel = __ballot_sync(kFull, need != 0);
-      while (sel) {
-        const int k = __ffs(sel) - 1;
-        sel &= sel - 1;
-        const uint32_t vk = __shfl_sync(kFull, v, k);
-        const unsigned long long nk = shfl64(need, k);
+    if (gtid == 0) {
+      ctl->any[(L + 2) & 3] = 0;
+      ctl->next[(pass + 2) & 3] = 0;
+    }
+    // heavy vertices' masks are set with atomics: cleared one level ahead
+    if (L + 2 < a.lcap)
+      for (uint64_t i = gtid; i < a.fs.nheavy; i += gthreads) nxt[(uint64_t)a.n + a.fs.heavy_list[i]] = 0ull;
+    bool my_any = false;
+    ms_tasks(&ctl->next[pass & 3], (uint64_t)a.fs.ntiles + nchunks, [&](uint32_t t) {
+      if (t < a.fs.ntiles) {
+        const uint2 tv = a.fs.tiles[t];
+        // a heavy vertex's level-L sources join its visited mask here (its
+        // other tiles add cur themselves, whichever of the two they read)
+        const unsigned long long seen = a.visit[tv.x] | cur[tv.x];
+        if (tv.y == 0 && lane == 0) a.visit[tv.x] = seen;
+        const unsigned long long need = ~seen & active;
+        if (!need) return;
+        const uint64_t vb = ldg(a.in_offs + tv.x), ve = ldg(a.in_offs + tv.x + 1);
+        const uint64_t b = vb + (uint64_t)tv.y * a.fs.tile, e = min(ve, b + a.fs.tile);
         double sA = 0.0, sB = 0.0;
-        const unsigned long long acc =
-            ms_forward_range(a, cur, nk, ldg(a.in_offs + vk), ldg(a.in_offs + vk + 1), sA, sB);
+        const unsigned long long acc = ms_range(a.rows, a.in_col, cur, need, b, e, sA, sB);
         if (acc) {
-          if (lane == 0) nxt[vk] = acc;
-          double* row = a.sigma + (uint64_t)vk * 64;
-          if ((acc >> lane) & 1ull) row[lane] = sA;
-          if ((acc >> (lane + 32)) & 1ull) row[lane + 32] = sB;
+          my_any = true;
+          if (lane == 0) atomicOr(&nxt[tv.x], acc);
+          double* row = a.rows + (uint64_t)tv.x * 64;
+          if ((acc >> lane) & 1ull) atomicAdd(&row[lane], sA);
+          if ((acc >> (lane + 32)) & 1ull) atomicAdd(&row[lane + 32], sB);
+        }
+        return;
+      }
+      const uint64_t first = (uint64_t)(t - a.fs.ntiles) << 5, v = first + lane;
+      uint64_t b = 0;
+      uint32_t d = 0;
+      bool light = false;
+      unsigned long long need = 0, seen = 0, mine = 0;
+      if (v < a.n) {
+        b = ldg(a.in_offs + v);
+        const uint64_t dd = ldg(a.in_offs + v + 1) - b;
+        light = dd <= a.fs.heavy;
+        if (light) {
+          seen = a.visit[v];
+          need = ~seen & active;
+          d = need ? (uint32_t)dd : 0u;
         }
       }
+      ms_chunk(a.rows, a.in_col, cur, need, b, d, [&](uint32_t o, unsigned long long acc, double sA, double sB) {
+        double* row = a.rows + (first + o) * 64;
+        if ((acc >> lane) & 1ull) row[lane] = sA;
+        if ((acc >> (lane + 32)) & 1ull) row[lane + 32] = sB;
+        if (lane == o) mine = acc;
+      });
+      if (light) {
+        nxt[v] = mine;
+        if (mine) a.visit[v] = seen | mine;
+      }
+      my_any |= mine != 0;
     });
-    for (uint64_t t = gwarp; t < a.fs.ntiles; t += nwarps) {
-      const uint2 tv = a.fs.tiles[t];
-      const unsigned long long need = ~a.visit[tv.x] & active;
-      if (!need) continue;
-      const uint64_t vb = ldg(a.in_offs + tv.x), ve = ldg(a.in_offs + tv.x + 1);
-      const uint64_t b = vb + (uint64_t)tv.y * a.fs.tile, e = min(ve, b + a.fs.tile);
-      double sA = 0.0, sB = 0.0;
-      const unsigned long long acc = ms_forward_range(a, cur, need, b, e, sA, sB);
-      if (acc) {
-        if (lane == 0) atomicOr(&nxt[tv.x], acc);
-        double* row = a.sigma + (uint64_t)tv.x * 64;
-        if ((acc >> lane) & 1ull) atomicAdd(&row[lane], sA);
-        if ((acc >> (lane + 32)) & 1ull) atomicAdd(&row[lane + 32], sB);
-      }
-    }
-    if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-    bool my_any = false;
-    for (uint64_t v = gtid; v < a.n; v += gthreads) {
-      const unsigned long long x = nxt[v];
-      if (x) {
-        a.visit[v] |= x;
-        my_any = true;
-      }
-    }
-    if (__any_sync(kFull, my_any) && lane == 0) atomicOr(&ctl->any[L & 3], 1u);
+    if (__any_sync(kFull, my_any) && lane == 0 &&
+        *reinterpret_cast<volatile uint32_t*>(&ctl->any[L & 3]) == 0)
+      atomicOr(&ctl->any[L & 3], 1u);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     if (*reinterpret_cast<volatile uint32_t*>(&ctl->any[L & 3]) == 0) break;
   }
   const uint32_t nlev = L + 1;  // levels 0..L are non-empty
-  // ---- backward: dependencies, levels nlev-2 .. 1 (LevelStructs.h:147-183) --
-  for (int Lb = (int)nlev - 2; Lb >= 1; --Lb) {
+  // ---- backward: dependencies, levels nlev-2 .. 1 (LevelStructs.h:147-183);
+  // the last level has none and only turns sigma into 1 / sigma ---------------
+  for (int Lb = (int)nlev - 1; Lb >= 1; --Lb) {
+    ++pass;
+    const bool last = Lb == (int)nlev - 1;
     const unsigned long long* cur = a.lm + (uint64_t)Lb * a.n;
-    const unsigned long long* nextl = a.lm + (uint64_t)(Lb + 1) * a.n;
+    const unsigned long long* nextl = a.lm + (uint64_t)(Lb + 1) * a.n;  // not read at the last level
     double* const hcur = a.hacc + (uint64_t)(Lb & 1) * a.bs.nheavy * 64;
     double* const hoth = a.hacc + (uint64_t)((Lb + 1) & 1) * a.bs.nheavy * 64;
-    ms_for_light(a, a.bs, a.offs, gwarp, nwarps, [&](uint32_t v, bool light) {
-      const unsigned long long cv = light ? cur[v] : 0ull;
-      unsigned sel = __ballot_sync(kFull, cv != 0);
-      while (sel) {
-        const int k = __ffs(sel) - 1;
-        sel &= sel - 1;
-        const uint32_t vk = __shfl_sync(kFull, v, k);
-        const unsigned long long ck = shfl64(cv, k);
-        double dA = 0.0, dB = 0.0;
-        ms_backward_range(a, nextl, ck, ldg(a.offs + vk), ldg(a.offs + vk + 1), dA, dB);
-        const uint64_t r = (uint64_t)vk * 64;
-        double t = 0.0;
-        if ((ck >> lane) & 1ull) {
-          const float d = (float)(dA * a.sigma[r + lane]);
-          a.dep[r + lane] = d;
-          t += d;
-        }
-        if ((ck >> (lane + 32)) & 1ull) {
-          const float d = (float)(dB * a.sigma[r + lane + 32]);
-          a.dep[r + lane + 32] = d;
-          t += d;
-        }
-        t = warp_sum(t);
-        if (lane == 0) a.bc[vk] += t;
+    if (gtid == 0) ctl->next[(pass + 2) & 3] = 0;
+    // vertex v's dependency for its sources in m, from the sums of its
+    // successors' rows; its own row becomes (1 + dep) / sigma.  Returns the
+    // lane's share of the dependencies' sum.
+    auto finish = [&](uint64_t v, unsigned long long m, double dA, double dB) -> double {
+      double* row = a.rows + v * 64;
+      double t = 0.0;
+      if ((m >> lane) & 1ull) {
+        const double sg = row[lane];
+        const float d = (float)(dA * sg);
+        row[lane] = (1.0 + (double)d) / sg;
+        t += d;
       }
+      if ((m >> (lane + 32)) & 1ull) {
+        const double sg = row[lane + 32];
+        const float d = (float)(dB * sg);
+        row[lane + 32] = (1.0 + (double)d) / sg;
+        t += d;
+      }
+      return t;
+    };
+    const uint32_t ntiles = last ? 0u : a.bs.ntiles;
+    ms_tasks(&ctl->next[pass & 3], (uint64_t)ntiles + nchunks, [&](uint32_t t) {
+      if (t < ntiles) {
+        const uint2 tv = a.bs.tiles[t];
+        const unsigned long long cv = cur[tv.x];
+        if (!cv) return;
+        const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
+        const uint64_t b = vb + (uint64_t)tv.y * a.bs.tile, e = min(ve, b + a.bs.tile);
+        double dA = 0.0, dB = 0.0;
+        const unsigned long long acc = ms_range(a.rows, a.col, nextl, cv, b, e, dA, dB);
+        double* h = hcur + (uint64_t)a.hidx[tv.x] * 64;
+        if ((acc >> lane) & 1ull) atomicAdd(&h[lane], dA);
+        if ((acc >> (lane + 32)) & 1ull) atomicAdd(&h[lane + 32], dB);
+        return;
+      }
+      const uint64_t first = (uint64_t)(t - ntiles) << 5, v = first + lane;
+      const unsigned long long cv0 = v < a.n ? cur[v] : 0ull;
+      if (!__any_sync(kFull, cv0 != 0)) return;
+      uint64_t b = 0;
+      uint32_t d = 0;
+      unsigned long long cv = 0;
+      if (cv0) {
+        b = ldg(a.offs + v);
+        const uint64_t dd = ldg(a.offs + v + 1) - b;
+        if (dd <= a.bs.heavy) {
+          cv = cv0;
+          d = last ? 0u : (uint32_t)dd;
+        }
+      }
+      double mine = 0.0;
+      bool did = false;
+      auto done = [&](uint32_t o, double dA, double dB) {
+        const double t2 = warp_sum(finish(first + o, shfl64(cv, o), dA, dB));
+        if (lane == o) {
+          mine = t2;
+          did = true;
+        }
+      };
+      ms_chunk(a.rows, a.col, nextl, cv, b, d,
+               [&](uint32_t o, unsigned long long, double dA, double dB) { done(o, dA, dB); });
+      // vertices without a successor on a shortest path: no dependency
+      for (unsigned rest = __ballot_sync(kFull, cv != 0 && !did); rest; rest &= rest - 1) {
+        const uint32_t o = __ffs(rest) - 1;
+        finish(first + o, shfl64(cv, o), 0.0, 0.0);
+      }
+      if (mine != 0.0) a.bc[v] += mine;
     });
-    for (uint64_t t = gwarp; t < a.bs.ntiles; t += nwarps) {
-      const uint2 tv = a.bs.tiles[t];
-      const unsigned long long cv = cur[tv.x];
-      if (!cv) continue;
-      const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
-      const uint64_t b = vb + (uint64_t)tv.y * a.bs.tile, e = min(ve, b + a.bs.tile);
-      double dA = 0.0, dB = 0.0;
-      ms_backward_range(a, nextl, cv, b, e, dA, dB);
-      double* h = hcur + (uint64_t)a.hidx[tv.x] * 64;
-      if ((cv >> lane) & 1ull) atomicAdd(&h[lane], dA);
-      if ((cv >> (lane + 32)) & 1ull) atomicAdd(&h[lane + 32], dB);
-    }
-    if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
+    if (!last && !grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     for (uint64_t i = gwarp; i < a.bs.nheavy; i += nwarps) {
       const uint32_t v = a.bs.heavy_list[i];
       // clear what level Lb+1 left in the other half (level Lb-1 adds there)
-      const unsigned long long prev = nextl[v];
+      const unsigned long long prev = last ? 0ull : nextl[v];
       if (prev) {
         double* ho = hoth + i * 64;
         if ((prev >> lane) & 1ull) ho[lane] = 0.0;
@@ -303,20 +401,8 @@ __global__ void __launch_bounds__(kBcBlock) ms_persistent(MsArgs a) {
       const unsigned long long cv = cur[v];
       if (!cv) continue;
       const double* h = hcur + i * 64;
-      const uint64_t r = (uint64_t)v * 64;
-      double t = 0.0;
-      if ((cv >> lane) & 1ull) {
-        const float d = (float)(h[lane] * a.sigma[r + lane]);
-        a.dep[r + lane] = d;
-        t += d;
-      }
-      if ((cv >> (lane + 32)) & 1ull) {
-        const float d = (float)(h[lane + 32] * a.sigma[r + lane + 32]);
-        a.dep[r + lane + 32] = d;
-        t += d;
-      }
-      t = warp_sum(t);
-      if (lane == 0) a.bc[v] += t;
+      const double t = warp_sum(finish(v, cv, h[lane], h[lane + 32]));
+      if (lane == 0 && t != 0.0) a.bc[v] += t;
     }
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
   }
@@ -605,7 +691,7 @@ int run_bc(gb_graph* g, const uint32_t* srcs_in, uint32_t nsrc, uint32_t batch, 
     for (int attempt = 0;; ++attempt) {
       const size_t need = carve_size<BcCtl>(1) + carve_size<double>(n) + carve_size<unsigned long long>((size_t)lcap * n) +
                           carve_size<unsigned long long>(n) + carve_size<double>((size_t)n * 64) +
-                          carve_size<float>((size_t)n * 64) + carve_size<double>(2 * (size_t)sched.nheavy * 64 + 1) +
+                          carve_size<double>(2 * (size_t)sched.nheavy * 64 + 1) +
                           carve_size<uint32_t>(n) + carve_size<uint32_t>(64) + (out_dev ? 0 : carve_size<float>(n));
       st = ws_reserve(g, need, s);
       if (st != GB_OK) return st;
@@ -616,8 +702,7 @@ int run_bc(gb_graph* g, const uint32_t* srcs_in, uint32_t nsrc, uint32_t batch, 
       a.bc = bc64;
       a.lm = cv.take<unsigned long long>((size_t)lcap * n);
       a.visit = cv.take<unsigned long long>(n);
-      a.sigma = cv.take<double>((size_t)n * 64);
-      a.dep = cv.take<float>((size_t)n * 64);
+      a.rows = cv.take<double>((size_t)n * 64);
       a.hacc = cv.take<double>(2 * (size_t)sched.nheavy * 64 + 1);
       a.hidx = cv.take<uint32_t>(n);
       uint32_t* dsrc = cv.take<uint32_t>(64);
@@ -630,7 +715,7 @@ int run_bc(gb_graph* g, const uint32_t* srcs_in, uint32_t nsrc, uint32_t batch, 
       a.srcs = dsrc;
       GB_CUDA(cudaMemsetAsync(bc64, 0, sizeof(double) * n, s));
       const void* kfn = reinterpret_cast<const void*>(&ms_persistent);
-      const int grid = coop_grid(g, kfn, kBcBlock, 0, t.blocks_per_sm);
+      const int grid = coop_grid(g, kfn, kMsBlock, 0, t.blocks_per_sm);
       if (grid <= 0) GB_FAIL(GB_ERR_CUDA, "gb_bc: cannot size cooperative grid");
       bool retry = false;
       total_ms = 0.0;
@@ -644,7 +729,7 @@ int run_bc(gb_graph* g, const uint32_t* srcs_in, uint32_t nsrc, uint32_t batch, 
         ms_seed<<<1, 32, 0, s>>>(a);
         void* args[] = {&a};
         KernelTimer kt(stats != nullptr, s);
-        GB_CUDA(cudaLaunchCooperativeKernel(kfn, grid, kBcBlock, args, 0, s));
+        GB_CUDA(cudaLaunchCooperativeKernel(kfn, grid, kMsBlock, args, 0, s));
         kt.stop(s);
         launches += 3;
         GB_CUDA(cudaMemcpyAsync(hc, a.ctl, sizeof(BcCtl), cudaMemcpyDeviceToHost, s));

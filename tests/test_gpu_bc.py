@@ -57,6 +57,30 @@ def test_bc_path_closed_form(cuda_device):
             assert np.allclose(got, [2.0 * v * (n - 1 - v) for v in range(n)], rtol=1e-6)
 
 
+@pytest.mark.parametrize("n,heavy,tile,nsrc", [(1, 16, 32, 2), (31, 4, 32, 31), (33, 8, 32, 33), (257, 16, 64, 64),
+                                               (4097, 128, 256, 65)])
+def test_bc_batched_edges(cuda_device, n, heavy, tile, nsrc):
+    """Chunk and tile remainders of the batched kernel: ragged vertex counts,
+    rows of exactly `heavy` and `heavy` + 1 arcs, a star whose hub spans
+    several tiles, vertices without a successor on a shortest path, repeated
+    sources, a last batch of one."""
+    rng = np.random.default_rng(n)
+    arcs = {(0, v) for v in range(1, n)} if n < 300 else set()
+    for k, d in enumerate((heavy, heavy + 1, tile + heavy, 2 * tile + 1)):
+        if n > d + k + 2:
+            arcs |= {(k + 1, int(v)) for v in rng.choice(np.arange(k + 2, n), d, replace=False)}
+    arcs |= {(v, v + 1) for v in range(n // 2, n - 1)}
+    src = [a for a, b in arcs] + [b for a, b in arcs]
+    dst = [b for a, b in arcs] + [a for a, b in arcs]
+    g = HostCSR.from_edges(n, src, dst)
+    srcs = rng.integers(0, n, nsrc).astype(np.uint32)
+    want = oracle.bc_level(g, srcs, f64=True)
+    for order in (0, 1):
+        with DeviceGraph(g, symmetric=True, reorder=order) as dg:
+            dg.set_tuning(heavy_degree=heavy, tile_edges=tile)
+            assert close(dg.bc(srcs, batch=64), want) < 1e-6
+
+
 def test_bc_directed_single_source_and_errors(cuda_device):
     g, perm = rmat(10, 8, seed=2, symmetrize=False)
     srcs = np.array([perm[0], perm[1], perm[2]], np.uint32)
