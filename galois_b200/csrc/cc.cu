@@ -28,6 +28,7 @@
 #include "device_common.cuh"
 #include "device_graph.cuh"
 #include "sweep.cuh"
+#include "union_find.cuh"
 
 namespace gb {
 
@@ -61,33 +62,6 @@ __global__ void cc_init(uint32_t* p, uint32_t n) {
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v = tid; v < n; v += stride) p[v] = (uint32_t)v;
-}
-
-__device__ __forceinline__ uint32_t find_root(uint32_t* p, uint32_t x) {
-  uint32_t px = p[x];
-  while (px != x) {
-    const uint32_t ppx = p[px];
-    if (ppx != px) p[x] = ppx;  // path halving (benign race: ancestors only)
-    x = px;
-    px = ppx;
-  }
-  return x;
-}
-
-// Link the trees of a and b: larger root goes under the smaller (ECL-CC style).
-__device__ __forceinline__ void link(uint32_t* p, uint32_t a, uint32_t b) {
-  uint32_t ra = find_root(p, a), rb = find_root(p, b);
-  for (int guard = 0; ra != rb && guard < (1 << 20); ++guard) {
-    if (ra < rb) {
-      const uint32_t ret = atomicCAS(&p[rb], rb, ra);
-      if (ret == rb) break;
-      rb = find_root(p, ret);
-    } else {
-      const uint32_t ret = atomicCAS(&p[ra], ra, rb);
-      if (ret == ra) break;
-      ra = find_root(p, ret);
-    }
-  }
 }
 
 __device__ __forceinline__ void compress_all(CcArgs& a, uint64_t gtid, uint64_t gthreads) {

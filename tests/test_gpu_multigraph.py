@@ -41,6 +41,21 @@ def test_multigraph_matches_per_graph_oracle(cuda_device):
         assert np.array_equal(lv2, expected(graphs, local2)[0])
 
 
+@pytest.mark.parametrize("sizes", [[1], [1, 1, 1], [31, 33, 1, 64], [5] * 100, [2000, 1, 3]])
+def test_multigraph_labels_from_levels(cuda_device, sizes):
+    """Labels taken from the BFS levels: graphs smaller than a warp's chunk, a
+    source in the giant component, in a small one (the giant is unreached) and
+    without arcs; labels asked for alone take the other path."""
+    graphs = [erdos_renyi(n, 3.0, seed=i) for i, n in enumerate(sizes)]
+    packed, first = pack_graphs(graphs)
+    for pick in (np.argmax, np.argmin, lambda d: len(d) // 2):
+        local = np.array([int(pick(g.degrees())) for g in graphs], np.uint32)
+        want_lv, want_lb = expected(graphs, local)
+        with DeviceGraph(packed, symmetric=True) as dg:
+            lv, lb = dg.multi_graph_bfs_cc(first, local)
+            assert np.array_equal(lv, want_lv) and np.array_equal(lb, want_lb)
+
+
 def test_multigraph_rejects_crossing_arcs_and_bad_sources(cuda_device):
     graphs = make_graphs(4, seed=1)
     packed, first = pack_graphs(graphs)
