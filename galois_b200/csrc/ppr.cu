@@ -13,13 +13,21 @@
 // B200 design: B right-hand sides stored vertex-major [n][B] so that, for
 // B = 128, one arc's gather is a single coalesced 512-byte row (a float4 per
 // lane) and the graph (column id + normalised weight, 8 bytes per arc) is
-// read once per iteration for all B columns.  One warp owns a row (light
-// rows); rows above `heavy` arcs are split into tiles whose partial rows meet
-// in a per-heavy-row accumulator.  The forward pulls over the in-arcs of the
-// device transpose, the adjoint over the out-arcs of the CSR.  Each solve is
+// read once per iteration for all B columns.  With fewer columns a row takes
+// fewer lanes (B / 4, rounded up to a power of two) and the warp takes that
+// many more arcs at once.  A warp takes the rows of a task one after another,
+// the next row's column ids and weights already loaded, eight 512-byte rows in
+// flight; rows above the tile size are split into tiles whose partial rows
+// are stored and then summed in arc order (the same result every time).  The forward pulls over the in-arcs of
+// the device transpose, the adjoint over the out-arcs of the CSR; a row
+// without arcs keeps its starting value and is not visited.  Each solve is
 // one cooperative persistent launch; per-column L1 changes are reduced per
 // block in shared memory and across blocks with fp64 atomics.  B = 1 (the
 // plain single-vector solve) uses lanes over arcs instead of columns.
+// RMAT-20, B = 128 (82 forward and 91 adjoint iterations): with tasks of up to
+// 1024 arcs, four rows in flight and no loads ahead of the row, forward plus
+// adjoint took 270 ms (a third of the warps' time waiting at the barriers);
+// this takes 193 ms, 1.07 ms an iteration or 7.6 TB/s of gathered rows.
 
 #include <algorithm>
 #include <vector>
@@ -37,14 +45,24 @@ namespace {
 
 constexpr int kPprBlock = 256;
 constexpr int kPprWarps = kPprBlock / 32;
-constexpr uint32_t kPprHeavy = 1024;  // arcs per row above which a row is tiled
-constexpr uint32_t kPprTile = 512;
+
+// Arcs per tile, and per row above which a row is tiled: a sixteenth to an
+// eighth of a warp's share of the arcs, so that the longest task ends with the
+// others, from 32 (a small graph's iteration lasts as long as its longest
+// task: 4 steps of gathers) to 512 (the partial rows stay under 1 byte per
+// arc and column).
+uint32_t ppr_tile(const gb_graph* g) {
+  const uint64_t share = g->m / ((uint64_t)g->sm_count * 32);
+  uint32_t t = 32;
+  while (t < 512 && 16ull * t <= share) t *= 2;
+  return t;
+}
 
 struct RowSched {
   uint2* tiles = nullptr;
   uint32_t* heavy = nullptr;
-  uint32_t* hidx = nullptr;  // [n] heavy index of a heavy row
   uint32_t ntiles = 0, nheavy = 0;
+  uint32_t tile = 0;  // arcs per tile; a row of more is heavy
 };
 
 struct PprState {
@@ -53,10 +71,9 @@ struct PprState {
   float* wn = nullptr;    // [m] w / s_src, CSR order
   float* wn_t = nullptr;  // [m] the same, transpose order
   uint32_t* flags = nullptr;  // [n/32] rows with a non-zero source term
-  double* l1 = nullptr;       // [3][128] per-column L1 change ring
+  double* l1 = nullptr;       // [3][128] per-column L1 change ring, then [128] ppr_seed's non-finite columns
   double* colnorm = nullptr;  // [128] per-column L1 norm of the adjoint's source term
-  float* hacc = nullptr;      // [max(nheavy)][128]
-  size_t hacc_rows = 0;
+  float* part = nullptr;      // [max(ntiles)][128] partial rows of the heavy rows' tiles
 };
 
 void free_state(gb_graph* g) {
@@ -65,7 +82,6 @@ void free_state(gb_graph* g) {
   for (RowSched* r : {&st->fwd, &st->bwd}) {
     cudaFree(r->tiles);
     cudaFree(r->heavy);
-    cudaFree(r->hidx);
   }
   cudaFree(st->s);
   cudaFree(st->wn);
@@ -73,16 +89,10 @@ void free_state(gb_graph* g) {
   cudaFree(st->flags);
   cudaFree(st->l1);
   cudaFree(st->colnorm);
-  cudaFree(st->hacc);
+  cudaFree(st->part);
   delete st;
   g->ppr_state = nullptr;
   g->ppr_free = nullptr;
-}
-
-__global__ void fill_hidx(const uint32_t* __restrict__ heavy, uint32_t nheavy, uint32_t* hidx) {
-  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = tid; i < nheavy; i += stride) hidx[heavy[i]] = (uint32_t)i;
 }
 
 // s_j = sum of out-arc weights; wn[e] = w[e] / s_j (one warp per row j)
@@ -109,9 +119,11 @@ __global__ void ppr_permute(const float* __restrict__ wn, const uint64_t* __rest
   for (uint64_t e = tid; e < m; e += stride) wn_t[e] = wn[emap[e]];
 }
 
-// flags[r] = 1 if row r of src has a non-zero entry; dst = scale * src
+// flags[r] = 1 if row r of src has a non-zero entry; both iterates start as
+// scale * src (rows without arcs stay so).  A column with a value that is not
+// finite never converges, wherever its row: bad[column] becomes NaN.
 __global__ void ppr_seed(const float* __restrict__ src, float scale, uint32_t n, uint32_t B, uint32_t* flags,
-                         float* __restrict__ dst) {
+                         float* __restrict__ dst, float* __restrict__ dst2, double* bad) {
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t lane = lane_id();
@@ -120,7 +132,8 @@ __global__ void ppr_seed(const float* __restrict__ src, float scale, uint32_t n,
     for (uint32_t b = lane; b < B; b += 32) {
       const float v = src[r * B + b];
       nz |= v != 0.f;
-      dst[r * B + b] = scale * v;
+      dst[r * B + b] = dst2[r * B + b] = scale * v;
+      if (!isfinite(v)) bad[b] = nan("");
     }
     nz = __any_sync(kFull, nz);
     if (lane == 0 && nz) atomicOr(&flags[r >> 5], 1u << (r & 31));
@@ -145,8 +158,8 @@ struct IterArgs {
   float alpha, tol;
   uint32_t max_iter;
   RowSched sched;
-  float* hacc;  // [nheavy][128]
-  double* l1;   // [3][128]
+  float* part;  // [ntiles][B]
+  double* l1;   // [3][128], then [128]: NaN for a column whose source term has a non-finite value
   const double* col_scale;  // per-column stopping scale (nullptr: 1)
   IterCtl* ctl;
 };
@@ -155,137 +168,243 @@ __device__ __forceinline__ float4 f4_fma(float a, float4 x, float4 y) {
   return make_float4(fmaf(a, x.x, y.x), fmaf(a, x.y, y.y), fmaf(a, x.z, y.z), fmaf(a, x.w, y.w));
 }
 
-// Sum over arcs [b, e) of wn * x[col] for this lane's 4 columns (WIDE) or, in
-// narrow mode (B == 1), for the whole warp (lanes over arcs, result in every
-// lane after the reduction).
-template <bool WIDE>
-__device__ __forceinline__ float4 row_sum(const IterArgs& a, const float* __restrict__ x, uint64_t b, uint64_t e) {
-  const uint32_t lane = lane_id();
+// A batch of arcs of one row: lane l holds the column id (and weight) of the
+// row's arc l, or of none.
+struct ArcLoad {
+  uint32_t c;
+  float w;
+};
+
+__device__ __forceinline__ ArcLoad load_arcs(const uint32_t* __restrict__ col, const float* __restrict__ wn, uint64_t b,
+                                             uint64_t e) {
+  ArcLoad r{0u, 0.f};
+  const uint64_t k = b + lane_id();
+  if (k < e) {
+    r.c = ldg(col + k);
+    if (wn) r.w = ldg(wn + k);
+  }
+  return r;
+}
+
+// Rows of B floats handled by LPA lanes (4 columns each), G = 32 / LPA arcs
+// per step, U steps in flight: 8 rows of 512 bytes at B = 128, at least two
+// steps at small B.
+template <int LPA>
+struct Wide {
+  static constexpr int G = 32 / LPA;
+  static constexpr int U = 8 / G > 2 ? 8 / G : 2;
+};
+
+// Sum over arcs [b, e) of wn * x[col] for this lane's 4 columns; `first` holds
+// the row's first 32 arcs.  Every group of LPA lanes returns the whole sum.
+template <int LPA>
+__device__ __forceinline__ float4 row_sum(const IterArgs& a, const float* __restrict__ x, uint64_t b, uint64_t e,
+                                          ArcLoad m) {
+  constexpr int G = Wide<LPA>::G, U = Wide<LPA>::U;
+  const uint32_t lane = lane_id(), sub = lane % LPA, grp = lane / LPA;
+  const bool act = 4 * sub < a.B;
+  const float* __restrict__ xs = x + 4 * sub;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (WIDE) {
-    const bool act = 4 * lane < a.B;
-    for (uint64_t k0 = b; k0 < e; k0 += 32) {
-      const uint32_t cnt = (uint32_t)(e - k0 < 32 ? e - k0 : 32);
-      uint32_t mc = 0;
-      float mw = 0.f;
-      if (lane < cnt) {
-        mc = ldg(a.col + k0 + lane);
-        mw = ldg(a.wn + k0 + lane);
+  for (uint64_t k0 = b; k0 < e; k0 += 32) {
+    const uint32_t cnt = (uint32_t)(e - k0 < 32 ? e - k0 : 32);
+    const ArcLoad nm = load_arcs(a.col, a.wn, k0 + 32, e);
+    for (uint32_t u = 0; u < cnt; u += U * G) {
+      float4 v[U];
+      float w[U];
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        const uint32_t i = u + j * G + grp;
+        const uint32_t c = __shfl_sync(kFull, m.c, i & 31);
+        w[j] = __shfl_sync(kFull, m.w, i & 31);
+        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (act && i < cnt) v[j] = *reinterpret_cast<const float4*>(xs + (uint64_t)c * a.B);
+        else w[j] = 0.f;
       }
-      uint32_t u = 0;
-      for (; u + 4 <= cnt; u += 4) {
-        const uint32_t c0 = __shfl_sync(kFull, mc, u), c1 = __shfl_sync(kFull, mc, u + 1);
-        const uint32_t c2 = __shfl_sync(kFull, mc, u + 2), c3 = __shfl_sync(kFull, mc, u + 3);
-        const float w0 = __shfl_sync(kFull, mw, u), w1 = __shfl_sync(kFull, mw, u + 1);
-        const float w2 = __shfl_sync(kFull, mw, u + 2), w3 = __shfl_sync(kFull, mw, u + 3);
-        if (act) {
-          const float4 x0 = *reinterpret_cast<const float4*>(x + (uint64_t)c0 * a.B + 4 * lane);
-          const float4 x1 = *reinterpret_cast<const float4*>(x + (uint64_t)c1 * a.B + 4 * lane);
-          const float4 x2 = *reinterpret_cast<const float4*>(x + (uint64_t)c2 * a.B + 4 * lane);
-          const float4 x3 = *reinterpret_cast<const float4*>(x + (uint64_t)c3 * a.B + 4 * lane);
-          acc = f4_fma(w0, x0, acc);
-          acc = f4_fma(w1, x1, acc);
-          acc = f4_fma(w2, x2, acc);
-          acc = f4_fma(w3, x3, acc);
-        }
-      }
-      for (; u < cnt; ++u) {
-        const uint32_t c0 = __shfl_sync(kFull, mc, u);
-        const float w0 = __shfl_sync(kFull, mw, u);
-        if (act) acc = f4_fma(w0, *reinterpret_cast<const float4*>(x + (uint64_t)c0 * a.B + 4 * lane), acc);
-      }
+#pragma unroll
+      for (int j = 0; j < U; ++j) acc = f4_fma(w[j], v[j], acc);
     }
-  } else {
-    float s = 0.f;
-    for (uint64_t k = b + lane; k < e; k += 32) s = fmaf(ldg(a.wn + k), x[ldg(a.col + k)], s);
-    acc.x = warp_sum(s);
+    m = nm;
+  }
+#pragma unroll
+  for (int o = LPA; o < 32; o <<= 1) {
+    acc.x += __shfl_xor_sync(kFull, acc.x, o);
+    acc.y += __shfl_xor_sync(kFull, acc.y, o);
+    acc.z += __shfl_xor_sync(kFull, acc.z, o);
+    acc.w += __shfl_xor_sync(kFull, acc.w, o);
   }
   return acc;
 }
 
-template <bool WIDE>
-__global__ void __launch_bounds__(kPprBlock) ppr_iterate(IterArgs a) {
-  __shared__ float s_diff[kPprWarps][128];
+// Calls fn(row, first arc, end, its first 32 arcs) for the rows of a task of
+// `rows` (a power of two, at most 32) consecutive rows that have between 1 and
+// `tile` arcs; the next row's arcs are loaded before fn runs.
+template <class Fn>
+__device__ __forceinline__ void ppr_rows(const uint64_t* __restrict__ offs, const uint32_t* __restrict__ col,
+                                         const float* __restrict__ wn, uint32_t n, uint64_t first, uint32_t rows,
+                                         uint32_t tile, Fn&& fn) {
+  const uint32_t lane = lane_id();
+  uint64_t rb = 0;
+  uint32_t rd = 0;
+  if (lane < rows && first + lane < n) {
+    rb = ldg(offs + first + lane);
+    const uint64_t d = ldg(offs + first + lane + 1) - rb;
+    rd = d <= tile ? (uint32_t)d : 0u;
+  }
+  unsigned todo = __ballot_sync(kFull, rd != 0);
+  if (!todo) return;
+  int k = __ffs(todo) - 1;
+  uint64_t b = __shfl_sync(kFull, rb, k), e = b + __shfl_sync(kFull, rd, k);
+  ArcLoad m = load_arcs(col, wn, b, e);
+  while (true) {
+    todo &= todo - 1;
+    int k2 = 0;
+    uint64_t b2 = 0, e2 = 0;
+    ArcLoad m2{0u, 0.f};
+    if (todo) {
+      k2 = __ffs(todo) - 1;
+      b2 = __shfl_sync(kFull, rb, k2), e2 = b2 + __shfl_sync(kFull, rd, k2);
+      m2 = load_arcs(col, wn, b2, e2);
+    }
+    fn((uint32_t)(first + k), b, e, m);
+    if (!todo) return;
+    k = k2, b = b2, e = e2, m = m2;
+  }
+}
+
+// Rows per task: 32, or fewer when there are too few rows for every warp.
+__device__ __forceinline__ uint32_t ppr_rows_per_task(uint32_t n, uint64_t nwarps) {
+  uint32_t r = 32;
+  while (r > 1 && (uint64_t)n < nwarps * r) r >>= 1;
+  return r;
+}
+
+// LPA: lanes per row of B floats; 0 for B = 1 (lanes over arcs).
+template <int LPA>
+__global__ void __launch_bounds__(kPprBlock, LPA ? 3 : 4) ppr_iterate(IterArgs a) {
+  constexpr bool WIDE = LPA != 0;
+  constexpr int L = WIDE ? LPA : 1;
+  __shared__ __align__(16) float s_diff[kPprWarps][128];  // written as float4
+  __shared__ float s_acc[kPprWarps][32];  // B = 1: row sums of a task
   IterCtl* ctl = a.ctl;
   const uint64_t deadline = kernel_deadline();
   const uint64_t gtid = blockIdx.x * (uint64_t)kPprBlock + threadIdx.x;
   const uint64_t gthreads = (uint64_t)gridDim.x * kPprBlock;
   const uint64_t gwarp = gtid >> 5, nwarps = gthreads >> 5;
   const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
-  const bool act = WIDE ? 4 * lane < a.B : lane == 0;
+  const bool act = WIDE ? (lane < L && 4 * lane < a.B) : lane == 0;  // lanes that write a row
+  const uint32_t tile = a.sched.tile;
+  const uint32_t rpt = WIDE ? ppr_rows_per_task(a.n, nwarps) : 32;
+  const uint64_t ntasks = a.sched.ntiles + ((uint64_t)a.n + rpt - 1) / rpt;
+  s_acc[wib][lane] = 0.f;
+  __syncwarp();
   for (uint32_t it = 0;; ++it) {
     const float* __restrict__ x = a.buf[it & 1];
     float* __restrict__ y = a.buf[(it + 1) & 1];
-    if (gtid == 0)
-      for (int c = 0; c < 128; ++c) a.l1[((it + 1) % 3) * 128 + c] = 0.0;
+    if (blockIdx.x == 0 && threadIdx.x < 128) a.l1[((it + 1) % 3) * 128 + threadIdx.x] = 0.0;
     float4 dsum = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto finish = [&](uint32_t r, float4 acc) {
+    auto finish = [&](uint32_t r, float4 acc, float4 o) {
       if (!act) return;
       const bool has_src = !a.flags || ((a.flags[r >> 5] >> (r & 31)) & 1u);
-      const uint64_t base = (uint64_t)r * a.B + (WIDE ? 4 * lane : 0);
-      if (WIDE) {
-        float4 v = make_float4(a.alpha * acc.x, a.alpha * acc.y, a.alpha * acc.z, a.alpha * acc.w);
-        if (has_src) v = f4_fma(a.src_scale, *reinterpret_cast<const float4*>(a.src + base), v);
-        const float4 o = *reinterpret_cast<const float4*>(x + base);
-        dsum.x += fabsf(v.x - o.x);
-        dsum.y += fabsf(v.y - o.y);
-        dsum.z += fabsf(v.z - o.z);
-        dsum.w += fabsf(v.w - o.w);
-        *reinterpret_cast<float4*>(y + base) = v;
-      } else {
-        float v = a.alpha * acc.x;
-        if (has_src) v = fmaf(a.src_scale, a.src[base], v);
-        dsum.x += fabsf(v - x[base]);
-        y[base] = v;
-      }
+      const uint64_t base = (uint64_t)r * a.B + 4 * lane;
+      float4 v = make_float4(a.alpha * acc.x, a.alpha * acc.y, a.alpha * acc.z, a.alpha * acc.w);
+      if (has_src) v = f4_fma(a.src_scale, *reinterpret_cast<const float4*>(a.src + base), v);
+      dsum.x += fabsf(v.x - o.x);
+      dsum.y += fabsf(v.y - o.y);
+      dsum.z += fabsf(v.z - o.z);
+      dsum.w += fabsf(v.w - o.w);
+      *reinterpret_cast<float4*>(y + base) = v;
     };
-    // light rows: one warp per row
-    for (uint64_t r = gwarp; r < a.n; r += nwarps) {
-      const uint64_t b = ldg(a.offs + r), e = ldg(a.offs + r + 1);
-      if (e - b > kPprHeavy) continue;
-      finish((uint32_t)r, row_sum<WIDE>(a, x, b, e));
-    }
-    // heavy rows: tiles of kPprTile arcs
-    for (uint64_t t = gwarp; t < a.sched.ntiles; t += nwarps) {
-      const uint2 tv = a.sched.tiles[t];
-      const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
-      const uint64_t b = vb + (uint64_t)tv.y * kPprTile, e = min(ve, b + kPprTile);
-      const float4 acc = row_sum<WIDE>(a, x, b, e);
-      float* h = a.hacc + (uint64_t)a.sched.hidx[tv.x] * 128 + (WIDE ? 4 * lane : 0);
-      if (act) {
-        atomicAdd(h, acc.x);
-        if (WIDE) {
-          atomicAdd(h + 1, acc.y);
-          atomicAdd(h + 2, acc.z);
-          atomicAdd(h + 3, acc.w);
+    auto finish1 = [&](uint32_t r, float acc) {
+      float v = a.alpha * acc;
+      if (!a.flags || ((a.flags[r >> 5] >> (r & 31)) & 1u)) v = fmaf(a.src_scale, a.src[r], v);
+      dsum.x += fabsf(v - x[r]);
+      y[r] = v;
+    };
+    auto old_row = [&](uint32_t r) {
+      return act ? *reinterpret_cast<const float4*>(x + (uint64_t)r * a.B + 4 * lane)
+                 : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    for (uint64_t t = gwarp; t < ntasks; t += nwarps) {
+      if (t < a.sched.ntiles) {  // one tile of a heavy row
+        const uint2 tv = a.sched.tiles[t];
+        const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
+        const uint64_t b = vb + (uint64_t)tv.y * tile, e = min(ve, b + tile);
+        float* h = a.part + t * a.B;
+        if constexpr (WIDE) {
+          const float4 acc = row_sum<L>(a, x, b, e, load_arcs(a.col, a.wn, b, e));
+          if (act) reinterpret_cast<float4*>(h)[lane] = acc;
+        } else {
+          float s = 0.f;
+          for (uint64_t k = b + lane; k < e; k += 32) s = fmaf(ldg(a.wn + k), x[ldg(a.col + k)], s);
+          s = warp_sum(s);
+          if (lane == 0) *h = s;
         }
+      } else if constexpr (WIDE) {
+        ppr_rows(a.offs, a.col, a.wn, a.n, (t - a.sched.ntiles) * rpt, rpt, tile,
+                 [&](uint32_t r, uint64_t b, uint64_t e, ArcLoad m) {
+                   const float4 o = old_row(r);  // in flight beside the gathers
+                   finish(r, row_sum<L>(a, x, b, e, m), o);
+                 });
+      } else {
+        // 32 rows' arcs walked together, four steps of loads in flight; a
+        // segmented sum per owner
+        const uint64_t r = ((t - a.sched.ntiles) << 5) + lane;
+        uint64_t b = 0;
+        uint32_t d = 0;
+        if (r < a.n) {
+          b = ldg(a.offs + r);
+          const uint64_t dd = ldg(a.offs + r + 1) - b;
+          d = dd <= tile ? (uint32_t)dd : 0u;
+        }
+        warp_expand_mlp<4, float>(
+            b, d, 0u, [&](bool valid, uint64_t e, uint32_t) { return valid ? ldg(a.col + e) : 0u; },
+            [&](bool valid, uint64_t e, uint32_t c, uint32_t) { return valid ? ldg(a.wn + e) * x[c] : 0.f; },
+            [&](bool valid, uint32_t owner, uint32_t, uint32_t, float v) {
+              const uint32_t key = valid ? owner : 0xFFFFFFFFu;
+#pragma unroll
+              for (int o = 1; o < 32; o <<= 1) {
+                const float w = __shfl_down_sync(kFull, v, o);
+                const uint32_t k2 = __shfl_down_sync(kFull, key, o);
+                if (lane + o < 32 && k2 == key) v += w;
+              }
+              const uint32_t kp = __shfl_up_sync(kFull, key, 1);
+              if (valid && (lane == 0 || kp != key)) s_acc[wib][owner] += v;
+              __syncwarp();
+            });
+        const float sum = s_acc[wib][lane];
+        s_acc[wib][lane] = 0.f;
+        __syncwarp();
+        if (d) finish1((uint32_t)r, sum);
       }
     }
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-    for (uint64_t i = gwarp; i < a.sched.nheavy; i += nwarps) {
-      const uint32_t r = a.sched.heavy[i];
-      float* h = a.hacc + i * 128 + (WIDE ? 4 * lane : 0);
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (act) {
-        acc.x = h[0];
-        h[0] = 0.f;
-        if (WIDE) {
-          acc.y = h[1];
-          acc.z = h[2];
-          acc.w = h[3];
-          h[1] = h[2] = h[3] = 0.f;
-        }
+    // heavy rows: their tiles follow one another from the one with k = 0
+    for (uint64_t t = gwarp; t < a.sched.ntiles; t += nwarps) {
+      const uint2 tv = a.sched.tiles[t];
+      if (tv.y != 0) continue;
+      const uint64_t d = ldg(a.offs + tv.x + 1) - ldg(a.offs + tv.x);
+      const uint32_t cnt = (uint32_t)((d + tile - 1) / tile);
+      if constexpr (WIDE) {
+        if (!act) continue;
+        const float4 o = old_row(tv.x);
+        const float4* h = reinterpret_cast<const float4*>(a.part + t * a.B) + lane;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (uint32_t k = 0; k < cnt; ++k) acc = f4_fma(1.f, h[(uint64_t)k * (a.B / 4)], acc);
+        finish(tv.x, acc, o);
+      } else {
+        float acc = 0.f;
+        for (uint32_t k = lane; k < cnt; k += 32) acc += a.part[t + k];
+        acc = warp_sum(acc);
+        if (lane == 0) finish1(tv.x, acc);
       }
-      finish(r, acc);
     }
     // per-column L1 change: block reduction, then one fp64 atomic per column
-    if (WIDE) {
-      s_diff[wib][4 * lane + 0] = dsum.x;
-      s_diff[wib][4 * lane + 1] = dsum.y;
-      s_diff[wib][4 * lane + 2] = dsum.z;
-      s_diff[wib][4 * lane + 3] = dsum.w;
-    } else if (lane == 0) {
-      s_diff[wib][0] = dsum.x;
+    if constexpr (WIDE) {
+      if (act) *reinterpret_cast<float4*>(&s_diff[wib][4 * lane]) = dsum;
+    } else {
+      dsum.x = warp_sum(dsum.x);
+      if (lane == 0) s_diff[wib][0] = dsum.x;
     }
     __syncthreads();
     if (threadIdx.x < a.B) {
@@ -293,15 +412,17 @@ __global__ void __launch_bounds__(kPprBlock) ppr_iterate(IterArgs a) {
       for (int w = 0; w < kPprWarps; ++w) sum += s_diff[w][threadIdx.x];
       if (sum != 0.f) atomicAdd(&a.l1[(it % 3) * 128 + threadIdx.x], (double)sum);
     }
-    __syncthreads();
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     // converged when every column's L1 change is at most tol (times the
-    // column's scale for the adjoint, whose source term is not normalised)
+    // column's scale for the adjoint, whose source term is not normalised):
+    // one thread per column
     bool done = true;
-    for (uint32_t c = 0; c < a.B; ++c) {
-      const double lim = (double)a.tol * (a.col_scale ? a.col_scale[c] : 1.0);
-      done &= *reinterpret_cast<volatile double*>(&a.l1[(it % 3) * 128 + c]) <= lim;
+    if (threadIdx.x < a.B) {
+      const double lim = (double)a.tol * (a.col_scale ? a.col_scale[threadIdx.x] : 1.0);
+      done = *reinterpret_cast<volatile double*>(&a.l1[(it % 3) * 128 + threadIdx.x]) + a.l1[3 * 128 + threadIdx.x] <=
+             lim;
     }
+    done = __syncthreads_and(done);
     if (gtid == 0) ctl->iters = it + 1;
     if (done || it + 1 >= a.max_iter) break;
   }
@@ -309,39 +430,62 @@ __global__ void __launch_bounds__(kPprBlock) ppr_iterate(IterArgs a) {
 
 // dL/dw for every arc of the CSR (rows = sources j):
 //   g[e] = alpha/s_j * sum_b x_j^b (lam_i^b - mu_j^b),  mu_j = (lam_j - gx_j)/alpha
-template <bool WIDE>
-__global__ void __launch_bounds__(kPprBlock) ppr_grad_w(const uint64_t* __restrict__ offs,
-                                                         const uint32_t* __restrict__ col, const float* __restrict__ s,
-                                                         const float* __restrict__ x, const float* __restrict__ lam,
-                                                         const float* __restrict__ gx, uint32_t n, uint32_t B,
-                                                         float alpha, RowSched sched, float* __restrict__ grad_w) {
+// Tasks as in ppr_iterate; the same number of lam rows in flight.
+template <int LPA>
+__global__ void __launch_bounds__(kPprBlock, LPA ? 3 : 4)
+    ppr_grad_w(const uint64_t* __restrict__ offs, const uint32_t* __restrict__ col, const float* __restrict__ s,
+               const float* __restrict__ x, const float* __restrict__ lam, const float* __restrict__ gx, uint32_t n,
+               uint32_t B, float alpha, RowSched sched, float* __restrict__ grad_w) {
+  constexpr bool WIDE = LPA != 0;
+  constexpr int L = WIDE ? LPA : 1;
   const uint64_t gtid = blockIdx.x * (uint64_t)kPprBlock + threadIdx.x;
   const uint64_t gwarp = gtid >> 5, nwarps = ((uint64_t)gridDim.x * kPprBlock) >> 5;
   const uint32_t lane = lane_id();
   const float inv_alpha = 1.0f / alpha;
-  auto run = [&](uint32_t j, uint64_t b, uint64_t e) {
+  auto run = [&](uint32_t j, uint64_t b, uint64_t e, ArcLoad m) {
     const float sj = s[j];
     const float scale = sj > 0.f ? alpha / sj : 0.f;
-    if (WIDE) {
-      const bool act = 4 * lane < B;
+    if constexpr (WIDE) {
+      constexpr int G = Wide<L>::G, U = Wide<L>::U;
+      const uint32_t sub = lane % L, grp = lane / L;
+      const bool act = 4 * sub < B;
+      const float* __restrict__ ls = lam + 4 * sub;
       float4 xj = make_float4(0.f, 0.f, 0.f, 0.f), mj = xj;
       if (act) {
-        const uint64_t base = (uint64_t)j * B + 4 * lane;
+        const uint64_t base = (uint64_t)j * B + 4 * sub;
         xj = *reinterpret_cast<const float4*>(x + base);
         const float4 lj = *reinterpret_cast<const float4*>(lam + base);
         const float4 gj = *reinterpret_cast<const float4*>(gx + base);
         mj = make_float4((lj.x - gj.x) * inv_alpha, (lj.y - gj.y) * inv_alpha, (lj.z - gj.z) * inv_alpha,
                          (lj.w - gj.w) * inv_alpha);
       }
-      for (uint64_t k = b; k < e; ++k) {
-        const uint32_t i = ldg(col + k);
-        float d = 0.f;
-        if (act) {
-          const float4 li = *reinterpret_cast<const float4*>(lam + (uint64_t)i * B + 4 * lane);
-          d = xj.x * (li.x - mj.x) + xj.y * (li.y - mj.y) + xj.z * (li.z - mj.z) + xj.w * (li.w - mj.w);
+      for (uint64_t k0 = b; k0 < e; k0 += 32) {
+        const uint32_t cnt = (uint32_t)(e - k0 < 32 ? e - k0 : 32);
+        const ArcLoad nm = load_arcs(col, nullptr, k0 + 32, e);
+        float out = 0.f;  // lane l: the gradient of arc k0 + l
+        for (uint32_t u = 0; u < cnt; u += U * G) {
+          float4 li[U];
+#pragma unroll
+          for (int q = 0; q < U; ++q) {
+            const uint32_t i = u + q * G + grp;
+            const uint32_t c = __shfl_sync(kFull, m.c, i & 31);
+            li[q] = mj;
+            if (act && i < cnt) li[q] = *reinterpret_cast<const float4*>(ls + (uint64_t)c * B);
+          }
+#pragma unroll
+          for (int q = 0; q < U; ++q) {
+            float d = xj.x * (li[q].x - mj.x) + xj.y * (li[q].y - mj.y) + xj.z * (li[q].z - mj.z) +
+                      xj.w * (li[q].w - mj.w);
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) d += __shfl_xor_sync(kFull, d, o);
+            // arc u + q * G + g is held by group g: hand it to its lane
+            const uint32_t at = lane - (u + q * G);  // wraps for lanes before it
+            const float got = __shfl_sync(kFull, d, (at * L) & 31);
+            if (at < (uint32_t)G) out = got;
+          }
         }
-        d = warp_sum(d);
-        if (lane == 0) grad_w[k] = scale * d;
+        if (lane < cnt) grad_w[k0 + lane] = scale * out;
+        m = nm;
       }
     } else {
       const float xj = x[j];
@@ -349,16 +493,49 @@ __global__ void __launch_bounds__(kPprBlock) ppr_grad_w(const uint64_t* __restri
       for (uint64_t k = b + lane; k < e; k += 32) grad_w[k] = scale * xj * (lam[ldg(col + k)] - mj);
     }
   };
-  for (uint64_t j = gwarp; j < n; j += nwarps) {
-    const uint64_t b = ldg(offs + j), e = ldg(offs + j + 1);
-    if (e - b > kPprHeavy) continue;
-    run((uint32_t)j, b, e);
+  const uint32_t rpt = ppr_rows_per_task(n, nwarps);
+  const uint64_t ntasks = sched.ntiles + ((uint64_t)n + rpt - 1) / rpt;
+  for (uint64_t t = gwarp; t < ntasks; t += nwarps) {
+    if (t < sched.ntiles) {
+      const uint2 tv = sched.tiles[t];
+      const uint64_t vb = ldg(offs + tv.x), ve = ldg(offs + tv.x + 1);
+      const uint64_t b = vb + (uint64_t)tv.y * sched.tile, e = min(ve, b + sched.tile);
+      run(tv.x, b, e, load_arcs(col, nullptr, b, e));
+    } else {
+      ppr_rows(offs, col, nullptr, n, (t - sched.ntiles) * rpt, rpt, sched.tile, run);
+    }
   }
-  for (uint64_t t = gwarp; t < sched.ntiles; t += nwarps) {
-    const uint2 tv = sched.tiles[t];
-    const uint64_t vb = ldg(offs + tv.x), ve = ldg(offs + tv.x + 1);
-    const uint64_t b = vb + (uint64_t)tv.y * kPprTile;
-    run(tv.x, b, min(ve, b + kPprTile));
+}
+
+// Lanes per row of B floats (0: one column).
+int lanes_per_row(uint32_t B) {
+  if (B == 1) return 0;
+  int l = 1;
+  while (4u * l < B) l *= 2;
+  return l;
+}
+
+const void* iterate_kernel(uint32_t B) {
+  switch (lanes_per_row(B)) {
+    case 0: return reinterpret_cast<const void*>(&ppr_iterate<0>);
+    case 1: return reinterpret_cast<const void*>(&ppr_iterate<1>);
+    case 2: return reinterpret_cast<const void*>(&ppr_iterate<2>);
+    case 4: return reinterpret_cast<const void*>(&ppr_iterate<4>);
+    case 8: return reinterpret_cast<const void*>(&ppr_iterate<8>);
+    case 16: return reinterpret_cast<const void*>(&ppr_iterate<16>);
+    default: return reinterpret_cast<const void*>(&ppr_iterate<32>);
+  }
+}
+
+const void* grad_kernel(uint32_t B) {
+  switch (lanes_per_row(B)) {
+    case 0: return reinterpret_cast<const void*>(&ppr_grad_w<0>);
+    case 1: return reinterpret_cast<const void*>(&ppr_grad_w<1>);
+    case 2: return reinterpret_cast<const void*>(&ppr_grad_w<2>);
+    case 4: return reinterpret_cast<const void*>(&ppr_grad_w<4>);
+    case 8: return reinterpret_cast<const void*>(&ppr_grad_w<8>);
+    case 16: return reinterpret_cast<const void*>(&ppr_grad_w<16>);
+    default: return reinterpret_cast<const void*>(&ppr_grad_w<32>);
   }
 }
 
@@ -395,24 +572,21 @@ int ensure_state(gb_graph* g, cudaStream_t s, PprState** out) {
     g->ppr_free = free_state;
     const uint32_t n = g->n;
     const uint64_t m = g->m;
-    rc = build_row_schedule(g->t_offs, n, m, kPprHeavy, kPprTile, g->sm_count, g->pinned, s, &st->fwd.tiles,
+    const uint32_t tile = ppr_tile(g);
+    st->fwd.tile = st->bwd.tile = tile;
+    rc = build_row_schedule(g->t_offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->fwd.tiles,
                             &st->fwd.heavy, &st->fwd.ntiles, &st->fwd.nheavy);
     if (rc != GB_OK) return rc;
-    rc = build_row_schedule(g->offs, n, m, kPprHeavy, kPprTile, g->sm_count, g->pinned, s, &st->bwd.tiles,
+    rc = build_row_schedule(g->offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->bwd.tiles,
                             &st->bwd.heavy, &st->bwd.ntiles, &st->bwd.nheavy);
     if (rc != GB_OK) return rc;
-    for (RowSched* r : {&st->fwd, &st->bwd}) {
-      GB_CUDA(cudaMalloc(&r->hidx, sizeof(uint32_t) * n));
-      if (r->nheavy) fill_hidx<<<g->sm_count, 256, 0, s>>>(r->heavy, r->nheavy, r->hidx);
-    }
-    st->hacc_rows = std::max<size_t>(1, std::max(st->fwd.nheavy, st->bwd.nheavy));
-    GB_CUDA(cudaMalloc(&st->hacc, sizeof(float) * 128 * st->hacc_rows));
-    GB_CUDA(cudaMemsetAsync(st->hacc, 0, sizeof(float) * 128 * st->hacc_rows, s));
+    const size_t ntiles = std::max<size_t>(1, std::max(st->fwd.ntiles, st->bwd.ntiles));
+    GB_CUDA(cudaMalloc(&st->part, sizeof(float) * 128 * ntiles));
     GB_CUDA(cudaMalloc(&st->s, sizeof(float) * n));
     GB_CUDA(cudaMalloc(&st->wn, sizeof(float) * std::max<uint64_t>(m, 1)));
     GB_CUDA(cudaMalloc(&st->wn_t, sizeof(float) * std::max<uint64_t>(m, 1)));
     GB_CUDA(cudaMalloc(&st->flags, sizeof(uint32_t) * ((n + 31) / 32)));
-    GB_CUDA(cudaMalloc(&st->l1, sizeof(double) * 3 * 128));
+    GB_CUDA(cudaMalloc(&st->l1, sizeof(double) * 4 * 128));
     GB_CUDA(cudaMalloc(&st->colnorm, sizeof(double) * 128));
   }
   *out = static_cast<PprState*>(g->ppr_state);
@@ -448,7 +622,7 @@ int solve(gb_graph* g, PprState* st, bool adjoint, uint32_t B, const float* src,
   a.alpha = alpha;
   a.tol = tol;
   a.max_iter = max_iter;
-  a.hacc = st->hacc;
+  a.part = st->part;
   a.l1 = st->l1;
   a.col_scale = adjoint ? st->colnorm : nullptr;
   a.ctl = ctl;
@@ -459,14 +633,15 @@ int solve(gb_graph* g, PprState* st, bool adjoint, uint32_t B, const float* src,
     ppr_colnorm<<<g->sm_count * 4, 256, 0, s>>>(src, g->n, B, st->colnorm);
   }
   GB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(IterCtl), s));
-  GB_CUDA(cudaMemsetAsync(st->l1, 0, sizeof(double) * 3 * 128, s));
+  GB_CUDA(cudaMemsetAsync(st->l1, 0, sizeof(double) * 4 * 128, s));
   GB_CUDA(cudaMemsetAsync(st->flags, 0, sizeof(uint32_t) * ((g->n + 31) / 32), s));
-  ppr_seed<<<g->sm_count * 8, 256, 0, s>>>(src, scale, g->n, B, st->flags, out);  // x0 = scale * src
+  ppr_seed<<<g->sm_count * 8, 256, 0, s>>>(src, scale, g->n, B, st->flags, out, tmp, st->l1 + 3 * 128);  // x0 = scale * src
   GB_CUDA(cudaGetLastError());
-  const bool wide = B > 1;
-  const void* kfn = wide ? reinterpret_cast<const void*>(&ppr_iterate<true>)
-                         : reinterpret_cast<const void*>(&ppr_iterate<false>);
-  const int grid = coop_grid(g, kfn, kPprBlock, 0, 0);
+  const void* kfn = iterate_kernel(B);
+  int grid = coop_grid(g, kfn, kPprBlock, 0, 0);
+  // no more CTAs than there is work for: every CTA takes part in the barriers
+  const uint64_t work = a.sched.ntiles + (B > 1 ? (uint64_t)g->n : ((uint64_t)g->n + 31) / 32);
+  grid = (int)std::min<uint64_t>(grid, (work + kPprWarps - 1) / kPprWarps);
   if (grid <= 0) GB_FAIL(GB_ERR_CUDA, "ppr: cannot size cooperative grid");
   void* args[] = {&a};
   KernelTimer kt(true, s);
@@ -564,12 +739,8 @@ extern "C" int gb_ppr_backward(gb_graph* g, uint32_t B, const float* x, const fl
   KernelTimer kt(stats != nullptr, s);
   if (grad_teleport) ppr_scale<<<g->sm_count * 8, 256, 0, s>>>(lam, 1.0f - alpha, nb, grad_teleport);
   if (grad_w) {
-    if (B > 1)
-      ppr_grad_w<true><<<g->sm_count * 8, kPprBlock, 0, s>>>(g->offs, g->col, st->s, x, lam, gx, g->n, B, alpha,
-                                                              st->bwd, grad_w);
-    else
-      ppr_grad_w<false><<<g->sm_count * 8, kPprBlock, 0, s>>>(g->offs, g->col, st->s, x, lam, gx, g->n, B, alpha,
-                                                               st->bwd, grad_w);
+    void* args[] = {&g->offs, &g->col, &st->s, &x, &lam, &gx, &g->n, &B, &alpha, &st->bwd, &grad_w};
+    GB_CUDA(cudaLaunchKernel(grad_kernel(B), g->sm_count * 8, kPprBlock, args, 0, s));
   }
   kt.stop(s);
   GB_CUDA(cudaGetLastError());

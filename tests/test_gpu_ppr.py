@@ -61,6 +61,44 @@ def test_forward_backward_vs_fp64(cuda_device, B):
         assert rel(gw.cpu().numpy(), gw_ref) < 1e-3
 
 
+@pytest.mark.parametrize("B", [1, 4, 8, 12, 20, 32, 36, 64, 68, 100])
+def test_row_and_tile_edges(cuda_device, B):
+    """Every lanes-per-row variant over rows of 0, 1, 7-9, 31-33 and 63-65
+    arcs (a small graph's tile is 32 arcs), a hub of many tiles and a ragged
+    vertex count; two runs give the same bits."""
+    import torch
+
+    from galois_b200.ppr import ppr
+
+    rng = np.random.default_rng(3)
+    n, src, dst = 517, [], []
+    for j, d in enumerate((0, 1, 7, 8, 9, 31, 32, 33, 63, 64, 65, 400)):
+        to = rng.choice(n, d, replace=False)
+        src += [j] * d + list(to)  # the same counts as out-rows and as in-rows
+        dst += list(to) + [j] * d
+    g = HostCSR.from_edges(n, src, dst)
+    assign_weights_f32(g, seed=4)
+    T = rng.random((n, B)).astype(np.float32) * (rng.random((n, B)) < 0.1)
+    T /= np.maximum(T.sum(0), 1e-30)
+    c = rng.standard_normal((n, B)).astype(np.float32)
+    w64 = g.w_f32.astype(np.float64)
+    x_ref = oppr.forward(g, T.astype(np.float64), w64, ALPHA)
+    gT_ref, gw_ref = oppr.backward(g, x_ref, c.astype(np.float64), w64, ALPHA)
+    runs = []
+    with DeviceGraph(g) as dg:
+        for _ in range(2):
+            Tt = torch.from_numpy(T).cuda().requires_grad_(True)
+            w = torch.from_numpy(g.w_f32).cuda().requires_grad_(True)
+            x = ppr(dg, Tt, w, ALPHA, 1e-7)
+            runs.append((x, *torch.autograd.grad((torch.from_numpy(c).cuda() * x).sum(), (Tt, w))))
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
+    x, gT, gw = (t.detach().cpu().numpy() for t in runs[0])
+    assert np.allclose(x, x_ref, atol=1e-6, rtol=1e-4)
+    assert rel(gT, gT_ref) < 1e-3
+    assert rel(gw, gw_ref) < 1e-3
+
+
 def test_heavy_rows_tiled(cuda_device):
     import torch
 
