@@ -33,9 +33,11 @@ enum DevErr : int {
 };
 
 struct GridBar {
-  unsigned int count;
+  unsigned int count;  // grid_barrier_last
   unsigned int gen;
-};
+  unsigned int word;  // grid_barrier: its top bit flips when every CTA has arrived
+};  // the kernel's error word follows (grid_barrier reads both with one load)
+static_assert(sizeof(GridBar) == 12, "GridBar and the error word behind it fill 16 bytes");
 
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
@@ -58,42 +60,58 @@ constexpr uint64_t kKernelBudgetNs = 60ull * 1000000000ull;
 
 __device__ __forceinline__ uint64_t kernel_deadline() { return globaltimer_ns() + kKernelBudgetNs; }
 
-// Grid-wide barrier for a cooperative launch of `nblocks` CTAs.  Returns false
-// (for every thread of the CTA) if the error word is set, the wait exceeded
-// `timeout_ns`, or the kernel passed `deadline`; callers then leave the kernel.
+// Grid-wide barrier for a cooperative launch of `nblocks` CTAs (1-D grid).
+// Returns false (for every thread of the CTA) if the error word is set, the
+// wait exceeded `timeout_ns`, or the kernel passed `deadline`; callers then
+// leave the kernel.  `bar` is 16-byte aligned and `err` the word behind it.
+//
+// What bounds it is the chain of L2 round trips, so a barrier is one atomic
+// and the polls of the same word: the CTAs of a phase add up to 2^31 (CTA 0
+// adds 2^31 - (nblocks - 1), the others 1), so the top bit flips with the last
+// arrival and the low bits are zero again.  The error word comes with each
+// poll (one 8-byte load: an error raised before any CTA's arrival is seen by
+// whoever sees the flip).  The arrival is a release and the fence after the
+// polls the matching acquire.  Measured on B200 against the count, the generation read before it
+// and the release store after it: 148 CTAs 2.4 -> 1.3 us, 592 3.1 -> 1.5 us,
+// 1184 4.2 -> 2.6 us, without the error read that was one more round trip.
 __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nblocks, int* err,
                                              uint64_t deadline = ~0ull,
                                              uint64_t timeout_ns = 2000000000ull) {
   __shared__ int s_ok;
   __syncthreads();
-  if (threadIdx.x == 0 && globaltimer_ns() > deadline) raise_err(err, kDevTimeout);
   if (threadIdx.x == 0) {
-    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> gen(bar->gen);
-    cuda::atomic_ref<unsigned int, cuda::thread_scope_device> cnt(bar->count);
-    const unsigned g = gen.load(cuda::memory_order_relaxed);
-    __threadfence();
-    const unsigned arrived = cnt.fetch_add(1u, cuda::memory_order_acq_rel);
+    if (blockIdx.x == 0 && globaltimer_ns() > deadline) raise_err(err, kDevTimeout);
+    const unsigned add = blockIdx.x == 0 ? 0x80000000u - (nblocks - 1) : 1u;
+    unsigned old;
+    unsigned long long now;  // the word, and the error word above it
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "l"(__cvta_generic_to_global(&bar->word)), "r"(add)
+                 : "memory");
     int ok = 1;
-    if (arrived == nblocks - 1) {
-      cnt.store(0u, cuda::memory_order_relaxed);
-      gen.fetch_add(1u, cuda::memory_order_release);
-    } else {
-      const uint64_t t0 = globaltimer_ns();
-      unsigned spins = 0;
-      while (gen.load(cuda::memory_order_acquire) == g) {
-        if ((++spins & 31u) == 0) {
-          if (read_err(err)) { ok = 0; break; }
-          if (globaltimer_ns() - t0 > timeout_ns) {
-            raise_err(err, kDevTimeout);
-            ok = 0;
-            break;
-          }
+    uint64_t t0 = 0;
+    for (unsigned spins = 1;; ++spins) {
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
+                   : "=l"(now)
+                   : "l"(__cvta_generic_to_global(&bar->word))
+                   : "memory");
+      if (now >> 32) {
+        ok = 0;
+        break;
+      }
+      if (((unsigned)now ^ old) >> 31) break;
+      __nanosleep(20);
+      if ((spins & 31u) == 0) {
+        const uint64_t t = globaltimer_ns();
+        if (!t0) t0 = t;
+        if (t - t0 > timeout_ns) {
+          raise_err(err, kDevTimeout);
+          ok = 0;
+          break;
         }
-        __nanosleep(40);
       }
     }
-    __threadfence();
-    if (ok && read_err(err)) ok = 0;
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
     s_ok = ok;
   }
   __syncthreads();
@@ -287,6 +305,38 @@ __device__ __forceinline__ void warp_expand_mlp(uint64_t beg, uint32_t deg, uint
     for (int k = 0; k < U; ++k) v2[k] = load2(valid[k], edge[k], v1[k], opl[k]);
 #pragma unroll
     for (int k = 0; k < U; ++k) consume(valid[k], pos[k], opl[k], v1[k], v2[k]);
+  }
+}
+
+// warp_expand that hands over U steps at once: fn(valid[U], edge[U]), by all
+// lanes, for callers whose work per step also waits on memory (atomics).
+template <int U, class Fn>
+__device__ __forceinline__ void warp_expand_all(uint64_t beg, uint32_t deg, Fn&& fn) {
+  const unsigned lane = lane_id();
+  uint32_t incl = deg;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, incl, o);
+    if ((int)lane >= o) incl += t;
+  }
+  const uint32_t total = __shfl_sync(kFull, incl, 31);
+  const uint64_t first = beg - (incl - deg);  // of the lane's vertex: edge = first + position
+  for (uint32_t base = 0; base < total; base += 32 * U) {
+    bool valid[U];
+    uint64_t edge[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const uint32_t e = base + 32 * k + lane;
+      uint32_t p = 0;
+#pragma unroll
+      for (uint32_t step = 16; step > 0; step >>= 1) {
+        const uint32_t v = __shfl_sync(kFull, incl, p + step - 1);
+        if (v <= e) p += step;
+      }
+      edge[k] = __shfl_sync(kFull, first, p) + e;
+      valid[k] = e < total;
+    }
+    fn(valid, edge);
   }
 }
 
