@@ -13,17 +13,19 @@
 //                    smaller with atomicMin, then every vertex jumps to its
 //                    root.  p[x] <= x always holds and sum(p) strictly drops
 //                    while anything changes, so it terminates with p = min id.
-//                    On a symmetric graph rounds after the first scan only
-//                    the vertices outside the sampled giant component.
+//                    On a symmetric graph the first round takes the first
+//                    two arcs of every row only (neighbour sampling, as
+//                    Afforest does), and the rounds after it scan in full the
+//                    rows outside the sampled giant component.
 //   GB_CC_UNIONFIND  one sweep of lock-free union-find (larger root linked
 //                    under the smaller with atomicCAS, path halving), then a
 //                    compression sweep.  Same labels.
 //   GB_CC_AFFOREST   neighbour sampling (first 2 arcs of every vertex), a
 //                    compression, detection of the most frequent root, then
 //                    union-find only over vertices outside that component.
-// On a symmetric graph each undirected edge is processed once (u > v) in a
-// full sweep; on a directed graph every arc is processed, giving weakly
-// connected components.
+// On a symmetric graph union-find processes each undirected edge once (u > v);
+// on a directed graph every arc is processed, giving weakly connected
+// components.
 
 #include "device_common.cuh"
 #include "device_graph.cuh"
@@ -48,8 +50,7 @@ struct CcArgs {
   const uint64_t* __restrict__ offs;
   const uint32_t* __restrict__ col;
   uint32_t n;
-  int half;    // process only u < v (symmetric graph)
-  int sorted;  // rows sorted ascending (relabelled graphs): a row's u < v arcs are its prefix
+  int half;    // symmetric graph
   uint32_t vend;  // rows from vend on are empty (degree-ordered graphs; else n)
   uint32_t* p;
   SweepSched sched;
@@ -104,24 +105,26 @@ __global__ void __launch_bounds__(BLOCK) cc_labelprop(CcArgs a) {
   const uint64_t gwarp = gtid >> 5, nwarps = gthreads >> 5;
   const uint32_t lane = lane_id();
   unsigned long long my_scanned = 0;
-  // After the first round (and its compression) every label is a root.  On a
-  // symmetric graph a later round then scans only the rows of vertices whose
+  // On a symmetric graph the first round hooks along each row's first two
+  // arcs: that joins most of a giant component (on a degree-ordered graph a
+  // row starts with its neighbours of highest degree) for a tenth of the arcs.
+  // RMAT-23 symmetric, degree order (259 M arcs): a first round over every
+  // arc u < v read 165 M arcs, 1.13 ms a call; this 0.41 ms.
+  // After a round's compression every label is a root.  A later round on a
+  // symmetric graph then scans only the rows of vertices whose
   // label is not the sampled giant label, each in full (both arc directions):
   // an arc whose ends disagree has at least one end outside the giant
   // component, and that end's row holds it (the skip Afforest makes,
   // applied to label propagation).  Most vertices join the giant component
-  // in the first round, so the confirming round reads few arcs.
+  // in the first round, so the later rounds read few arcs.
   uint32_t giant = 0xFFFFFFFFu;
   for (uint32_t r = 0;; ++r) {
     if (r >= a.max_rounds) {
       if (gtid == 0) raise_err(&ctl->err, kDevMaxRounds);
       break;
     }
+    const bool sampling = a.half && r == 0;
     const bool skip_giant = a.half && r >= 1;
-    // the first sweep of a symmetric graph takes each edge once, as its arc
-    // u < v: on a degree-ordered graph that is a prefix of a hub's row (its
-    // neighbours of higher degree), and the gathered labels are the hubs'
-    const bool all_dirs = !a.half || skip_giant;  // arcs u > v too
     uint32_t* changed = &ctl->changed[r % 3];
     if (gtid == 0) ctl->changed[(r + 1) % 3] = 0;
     bool my_change = false;
@@ -164,20 +167,16 @@ __global__ void __launch_bounds__(BLOCK) cc_labelprop(CcArgs a) {
     const uint64_t total = nchunks + a.sched.ntiles;
     // one tile of a heavy row: 8 column loads, then 8 label loads, per lane
     auto tile_fn = [&](uint32_t v, uint64_t b, uint64_t e) {
-      // a sorted row's u < v arcs end before the first u >= v
-      if (!all_dirs && a.sorted && ldg(a.col + b) >= v) return;  // warp-uniform
       const uint32_t pv = a.p[v];
       if (skip_giant && pv == giant) return;  // warp-uniform
       constexpr int UT = 8;
       for (uint64_t i0 = b; i0 < e; i0 += 32 * UT) {
-        if (i0 > b && !all_dirs && a.sorted && ldg(a.col + i0) >= v) break;  // warp-uniform
         if (lane == 0) my_scanned += e - i0 < 32 * UT ? e - i0 : (uint64_t)(32 * UT);  // the arcs read
         uint32_t u[UT], pu[UT];
 #pragma unroll
         for (int k = 0; k < UT; ++k) {
           const uint64_t i = i0 + lane + 32 * k;
-          const uint32_t x = i < e ? ldg(a.col + i) : 0u;
-          u[k] = (i < e && (all_dirs || x < v)) ? x : 0xFFFFFFFFu;
+          u[k] = i < e ? ldg(a.col + i) : 0xFFFFFFFFu;
         }
 #pragma unroll
         for (int k = 0; k < UT; ++k) pu[k] = u[k] != 0xFFFFFFFFu ? a.p[u[k]] : 0u;
@@ -185,7 +184,18 @@ __global__ void __launch_bounds__(BLOCK) cc_labelprop(CcArgs a) {
         for (int k = 0; k < UT; ++k) hook(u[k] != 0xFFFFFFFFu, pv, pu[k]);
       }
     };
-    for (uint64_t t = gwarp; t < total; t += nwarps) {
+    if (sampling) {
+      for (uint64_t v = gtid; v < a.vend; v += gthreads) {
+        const uint64_t b = ldg(a.offs + v), e = ldg(a.offs + v + 1);
+        const uint32_t u0 = b < e ? ldg(a.col + b) : (uint32_t)v, u1 = b + 1 < e ? ldg(a.col + b + 1) : (uint32_t)v;
+        const uint32_t p0 = a.p[u0], p1 = a.p[u1];
+        hook(true, (uint32_t)v, p0);
+        hook(true, (uint32_t)v, p1);
+        my_scanned += e - b < 2 ? e - b : 2;
+      }
+      my_change = true;  // the rest of the arcs are still to be looked at
+    }
+    for (uint64_t t = gwarp; t < total && !sampling; t += nwarps) {
       if (t < nchunks) {
         const uint64_t v64 = (t << 5) + lane;
         uint64_t b = 0;
@@ -206,10 +216,7 @@ __global__ void __launch_bounds__(BLOCK) cc_labelprop(CcArgs a) {
         my_scanned += d;
         warp_expand_mlp<4, uint32_t>(
             b, d, (uint32_t)v64,
-            [&](bool valid, uint64_t e, uint32_t v) {
-              const uint32_t u = valid ? ldg(a.col + e) : 0u;
-              return (valid && (all_dirs || u < v)) ? u : 0xFFFFFFFFu;
-            },
+            [&](bool valid, uint64_t e, uint32_t) { return valid ? ldg(a.col + e) : 0xFFFFFFFFu; },
             [&](bool, uint64_t, uint32_t u, uint32_t) { return u != 0xFFFFFFFFu ? a.p[u] : 0u; },
             [&](bool, uint32_t owner, uint32_t, uint32_t u, uint32_t pu) {
               const uint32_t opv = __shfl_sync(kFull, pv, owner);
@@ -235,6 +242,8 @@ __global__ void __launch_bounds__(BLOCK) cc_labelprop(CcArgs a) {
       if (blockIdx.x == 0) sample_giant<BLOCK>(a, ctl);
       if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
       giant = *reinterpret_cast<volatile uint32_t*>(&ctl->giant);
+    } else if (a.half) {
+      giant = *reinterpret_cast<volatile uint32_t*>(&a.p[giant]);  // the giant's root may have gone under another
     }
   }
   my_scanned = warp_sum(my_scanned);
@@ -322,7 +331,6 @@ int run_cc(gb_graph* g, int algo, uint32_t* label_out, gb_stats* stats, cudaStre
   a.col = g->col;
   a.n = n;
   a.half = g->symmetric ? 1 : 0;
-  a.sorted = (g->perm && g->order != GB_ORDER_DEGREE_UNSORTED && g->m < (1ull << 31)) ? 1 : 0;
   a.vend = g->perm ? std::max<uint32_t>(g->zero_from, 1u) : n;
   a.sched = sched;
   a.max_rounds = 1u << 20;
