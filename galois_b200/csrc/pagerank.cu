@@ -170,6 +170,86 @@ __device__ __forceinline__ bool seg_reduce(bool valid, uint32_t owner, float& x)
   return valid && (lane == 0 || kprev != key);
 }
 
+// Sums over the rows of a 32-row chunk whose lanes hold (first arc, arc
+// count): four rows at a time, eight lanes each, four columns per lane loaded
+// ahead of the four gathers, the next four rows' columns loading meanwhile.
+// Returns the lane's own row's sum.  Walking the chunk's arcs 32 at a time
+// (owner search and segmented sum, about 80 instructions per 32 arcs) was
+// bound by instruction issue; this takes about 20.  Pull-residual, RMAT-21
+// directed in file order (32 M arcs): 204 -> 174 us a round, 189 G arcs/s,
+// now about the rate of 4-byte gathers from L2.
+template <class Gather>
+__device__ __forceinline__ float chunk_row_sums(const uint32_t* __restrict__ col, uint64_t b, uint32_t d,
+                                                Gather&& gather) {
+  const uint32_t lane = lane_id(), sub = lane & 7u, grp = lane >> 3;
+  auto load = [&](uint64_t rb, uint32_t rd, uint32_t k, uint32_t (&u)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = k + 8 * j < rd ? ldg(col + rb + k + 8 * j) : 0xFFFFFFFFu;
+  };
+  float mine = 0.f;
+  uint64_t rb = __shfl_sync(kFull, b, grp);
+  uint32_t rd = __shfl_sync(kFull, d, grp);
+  uint32_t u[4];
+  load(rb, rd, sub, u);
+#pragma unroll 1
+  for (uint32_t q = 0; q < 8; ++q) {
+    const uint64_t nb = __shfl_sync(kFull, b, (4 * q + 4 + grp) & 31);
+    uint32_t nd = __shfl_sync(kFull, d, (4 * q + 4 + grp) & 31);
+    if (q == 7) nd = 0;
+    uint32_t un[4];
+    load(nb, nd, sub, un);
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (u[j] != 0xFFFFFFFFu) sum += gather(u[j]);
+    for (uint32_t k = sub + 32; k < rd; k += 32) {
+      load(rb, rd, k, u);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (u[j] != 0xFFFFFFFFu) sum += gather(u[j]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+    const float got = __shfl_sync(kFull, sum, (lane & 3u) * 8);
+    if ((lane >> 2) == q) mine = got;
+    rb = nb, rd = nd;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = un[j];
+  }
+  return mine;
+}
+
+// The sum over one tile [b, e) of a heavy row, by a warp (in every lane):
+// 8 column loads per lane per round, the next round's loads issued before
+// this round's gathers are summed.
+template <class Gather>
+__device__ __forceinline__ float tile_row_sum(const uint32_t* __restrict__ col, uint64_t b, uint64_t e,
+                                              Gather&& gather) {
+  const uint32_t lane = lane_id();
+  constexpr int UT = 8;
+  uint32_t u[UT];
+#pragma unroll
+  for (int k = 0; k < UT; ++k) {
+    const uint64_t i = b + lane + 32 * k;
+    u[k] = i < e ? ldg(col + i) : 0xFFFFFFFFu;
+  }
+  float sum = 0.f;
+  for (uint64_t i0 = b; i0 < e; i0 += 32 * UT) {
+    uint32_t un[UT];
+#pragma unroll
+    for (int k = 0; k < UT; ++k) {
+      const uint64_t i = i0 + 32 * UT + lane + 32 * k;
+      un[k] = i < e ? ldg(col + i) : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (int k = 0; k < UT; ++k) sum += u[k] != 0xFFFFFFFFu ? gather(u[k]) : 0.f;
+#pragma unroll
+    for (int k = 0; k < UT; ++k) u[k] = un[k];
+  }
+  return warp_sum(sum);
+}
+
 // Jacobi pull iterations, one cooperative persistent launch.  Shared memory
 // is kept small (one float per lane) so that the SM's unified L1/shared array
 // serves as L1 for the gathers; on a degree-ordered graph the hot
@@ -223,10 +303,8 @@ __device__ __forceinline__ void clear_change(PrCtl* ctl, uint32_t slot_set) {
   ctl->linf[slot_set] = 0u;
 }
 
-template <int BLOCK, int U, int MINB>
+template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_persistent(PrArgs a) {
-  constexpr int kW = BLOCK / 32;
-  __shared__ float s_acc[kW][32];
   __shared__ double s_l1, s_total;
   __shared__ uint32_t s_max;
   if (threadIdx.x == 0) {
@@ -239,9 +317,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_persistent(PrArgs a) {
   const uint64_t gtid = blockIdx.x * (uint64_t)BLOCK + threadIdx.x;
   const uint64_t gthreads = (uint64_t)gridDim.x * BLOCK;
   const uint64_t gwarp = gtid >> 5, nwarps = gthreads >> 5;
-  const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
-  s_acc[wib][lane] = 0.f;
-  __syncwarp();
+  const uint32_t lane = lane_id();
   for (uint32_t it = 0;; ++it) {
     const float* __restrict__ c_in = a.c[it & 1];
     float* __restrict__ c_out = a.c[(it + 1) & 1];
@@ -260,9 +336,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_persistent(PrArgs a) {
       my_l1 += (double)fabsf(value - old);
       my_max = fmaxf(my_max, fabsf(value - old));
     };
-    // Tasks: 32-vertex chunks (warp expansion, U steps of loads in flight;
-    // a chunk without arcs only finishes its vertices), then heavy-vertex
-    // tiles (sweep.cuh's decomposition).
+    // Tasks: 32-vertex chunks (a chunk without arcs only finishes its
+    // vertices), then heavy-vertex tiles (sweep.cuh's decomposition).
     const uint64_t nchunks = ((uint64_t)(it >= 2 ? a.zero_from : a.n) + 31) >> 5;  // constant tail skipped
     const uint64_t total = nchunks + a.sched.ntiles;
     for (uint64_t t = gwarp; t < total; t += nwarps) {
@@ -277,51 +352,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_persistent(PrArgs a) {
           heavy = dd > a.sched.heavy;
           d = heavy ? 0u : (uint32_t)dd;
         }
-        const uint32_t dmax = __reduce_max_sync(kFull, d);
-        if (dmax == 0) {
-          if (v < a.n && !heavy) finish((uint32_t)v, 0.f);
-        } else {
-          // U steps of (column id, contribution) loads in flight per lane
-          warp_expand_mlp<U, float>(
-              b, d, (uint32_t)v, [&](bool valid, uint64_t e, uint32_t) { return valid ? ldg(a.col + e) : 0u; },
-              [&](bool valid, uint64_t, uint32_t u, uint32_t) { return valid ? gather(u) : 0.f; },
-              [&](bool valid, uint32_t owner, uint32_t, uint32_t, float x) {
-                if (seg_reduce(valid, owner, x)) s_acc[wib][owner] += x;
-                __syncwarp();
-              });
-          const float sum = s_acc[wib][lane];
-          s_acc[wib][lane] = 0.f;
-          __syncwarp();
-          if (v < a.n && !heavy) finish((uint32_t)v, sum);
-        }
+        const float sum = __any_sync(kFull, d != 0) ? chunk_row_sums(a.col, b, d, gather) : 0.f;
+        if (v < a.n && !heavy) finish((uint32_t)v, sum);
       } else {
-        // one tile of a heavy row: 8 column loads per lane per round, the
-        // next round's loads issued before this round's gathers are summed
         const uint2 tv = a.sched.tiles[t - nchunks];
         const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
         const uint64_t b = vb + (uint64_t)tv.y * a.sched.tile;
-        const uint64_t e = min(ve, b + a.sched.tile);
-        constexpr int UT = 8;
-        uint32_t u[UT];
-#pragma unroll
-        for (int k = 0; k < UT; ++k) {
-          const uint64_t i = b + lane + 32 * k;
-          u[k] = i < e ? ldg(a.col + i) : 0xFFFFFFFFu;
-        }
-        float sum = 0.f;
-        for (uint64_t i0 = b; i0 < e; i0 += 32 * UT) {
-          uint32_t un[UT];
-#pragma unroll
-          for (int k = 0; k < UT; ++k) {
-            const uint64_t i = i0 + 32 * UT + lane + 32 * k;
-            un[k] = i < e ? ldg(a.col + i) : 0xFFFFFFFFu;
-          }
-#pragma unroll
-          for (int k = 0; k < UT; ++k) sum += u[k] != 0xFFFFFFFFu ? gather(u[k]) : 0.f;
-#pragma unroll
-          for (int k = 0; k < UT; ++k) u[k] = un[k];
-        }
-        sum = warp_sum(sum);
+        const float sum = tile_row_sum(a.col, b, min(ve, b + a.sched.tile), gather);
         if (lane == 0) atomicAdd(&acc_cur[tv.x], sum);
       }
     }
@@ -374,31 +411,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_flat(PrArgs a) {
     if (gtid == 0) clear_change(ctl, (it + 1) % 3);
     for (uint64_t t = gwarp; t < total; t += nwarps) {
       if (t < a.sched.ntiles) {
-        // one tile of a heavy row (as in pr_pull_persistent)
         const uint2 tv = a.sched.tiles[t];
         const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
         const uint64_t b = vb + (uint64_t)tv.y * a.sched.tile;
-        const uint64_t e = min(ve, b + a.sched.tile);
-        uint32_t u[UT];
-#pragma unroll
-        for (int k = 0; k < UT; ++k) {
-          const uint64_t i = b + lane + 32 * k;
-          u[k] = i < e ? ldg(a.col + i) : 0xFFFFFFFFu;
-        }
-        float sum = 0.f;
-        for (uint64_t i0 = b; i0 < e; i0 += 32 * UT) {
-          uint32_t un[UT];
-#pragma unroll
-          for (int k = 0; k < UT; ++k) {
-            const uint64_t i = i0 + 32 * UT + lane + 32 * k;
-            un[k] = i < e ? ldg(a.col + i) : 0xFFFFFFFFu;
-          }
-#pragma unroll
-          for (int k = 0; k < UT; ++k) sum += u[k] != 0xFFFFFFFFu ? c_in[u[k]] : 0.f;
-#pragma unroll
-          for (int k = 0; k < UT; ++k) u[k] = un[k];
-        }
-        sum = warp_sum(sum);
+        const float sum = tile_row_sum(a.col, b, min(ve, b + a.sched.tile), [&](uint32_t u) { return c_in[u]; });
         if (lane == 0) atomicAdd(&acc_cur[tv.x], sum);
       } else {
         // one run of 256 arcs of the light rows
@@ -733,70 +749,80 @@ __global__ void pr_resid_init(PrArgs a) {
   }
 }
 
-__global__ void __launch_bounds__(kBlock) pr_pull_residual_persistent(PrArgs a) {
-  __shared__ float s_acc[kWarps][32];
+// The vertex pass of pull-residual round it: closes round it - 1 (a positive
+// sum becomes the residual), then takes the residuals above tol (value +=
+// residual, delta = residual * alpha / outdeg) and counts those with out-arcs.
+__device__ __forceinline__ void resid_vertex_pass(const PrArgs& a, uint32_t it, const float* acc_prev, float* acc_cur,
+                                                  uint64_t gtid, uint64_t gthreads) {
+  uint32_t my_accum = 0;
+  for (uint64_t v = gtid; v < a.n; v += gthreads) {
+    float r = a.residual[v];
+    if (it > 0) {
+      const float sum = acc_prev[v];
+      if (sum > 0.f) r = sum;
+    }
+    // the sums of round it - 2, read by round it - 1: zeroed for this
+    // round's gather (zeroing the slots the last gather's atomics just
+    // updated stalls)
+    acc_cur[v] = 0.f;
+    float d = 0.f;
+    if (r > a.tol) {
+      a.value[v] += r;
+      const uint32_t k = a.nout[v];
+      if (k > 0) {
+        d = r * a.alpha / (float)k;
+        ++my_accum;
+      }
+      r = 0.f;
+    }
+    a.residual[v] = r;
+    a.delta[v] = d;
+  }
+  my_accum = __reduce_add_sync(kFull, my_accum);
+  if (lane_id() == 0 && my_accum) atomicAdd(&a.ctl->active[it % 3], my_accum);
+}
+
+// Pull-residual rounds over the rows as stored: the vertex pass, then every
+// row's sum of deltas (light rows stored, heavy rows' tiles added), two grid
+// barriers a round.  RMAT-21 directed (32 M arcs): see chunk_row_sums.
+__global__ void __launch_bounds__(kBlock, 6) pr_pull_residual_persistent(PrArgs a) {
   PrCtl* ctl = a.ctl;
   const uint64_t deadline = kernel_deadline();
   const uint64_t gtid = blockIdx.x * (uint64_t)kBlock + threadIdx.x;
   const uint64_t gthreads = (uint64_t)gridDim.x * kBlock;
   const uint64_t gwarp = gtid >> 5, nwarps = gthreads >> 5;
-  const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
-  s_acc[wib][lane] = 0.f;
-  __syncwarp();
+  const uint32_t lane = lane_id();
+  const uint64_t nchunks = ((uint64_t)a.n + 31) >> 5;
   for (uint32_t it = 0;; ++it) {
+    float* const acc_prev = (it & 1) ? a.acc : a.acc2;
+    float* const acc_cur = (it & 1) ? a.acc2 : a.acc;
     if (gtid == 0) ctl->active[(it + 1) % 3] = 0;
-    uint32_t my_accum = 0;
-    for (uint64_t v = gtid; v < a.n; v += gthreads) {
-      a.delta[v] = 0.f;
-      const float r = a.residual[v];
-      if (r > a.tol) {
-        a.residual[v] = 0.f;
-        a.value[v] += r;
-        const uint32_t k = a.nout[v];
-        if (k > 0) {
-          a.delta[v] = r * a.alpha / (float)k;
-          ++my_accum;
-        }
-      }
-    }
-    my_accum = __reduce_add_sync(kFull, my_accum);
-    if (lane == 0 && my_accum) atomicAdd(&ctl->active[it % 3], my_accum);
+    resid_vertex_pass(a, it, acc_prev, acc_cur, gtid, gthreads);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-    auto finish = [&](uint32_t v, float sum) {
-      if (sum > 0.f) a.residual[v] = sum;
+    auto gather = [&](uint32_t u) {
+      const float d = a.delta[u];
+      return d > 0.f ? d : 0.f;
     };
-    sweep_all(
-        a.offs, a.n, a.sched, gwarp, nwarps,
-        [&](bool valid, uint64_t e, uint32_t owner, uint32_t) {
-          float x = 0.f;
-          if (valid) {
-            const float d = a.delta[ldg(a.col + e)];
-            x = d > 0.f ? d : 0.f;
-          }
-          if (seg_reduce(valid, owner, x)) s_acc[wib][owner] += x;
-          __syncwarp();
-        },
-        [&](uint32_t v, bool valid, bool heavy) {
-          const float sum = s_acc[wib][lane];
-          s_acc[wib][lane] = 0.f;
-          __syncwarp();
-          if (valid && !heavy) finish(v, sum);
-        },
-        [&](uint32_t v, uint64_t b, uint64_t e) {
-          float s = 0.f;
-          for (uint64_t i = b + lane; i < e; i += 32) {
-            const float d = a.delta[ldg(a.col + i)];
-            s += d > 0.f ? d : 0.f;
-          }
-          s = warp_sum(s);
-          if (lane == 0) atomicAdd(&a.acc[v], s);
-        });
-    if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-    for (uint64_t i = gtid; i < a.sched.nheavy; i += gthreads) {
-      const uint32_t v = a.sched.heavy_list[i];
-      const float sum = a.acc[v];
-      a.acc[v] = 0.f;
-      finish(v, sum);
+    for (uint64_t t = gwarp; t < nchunks + a.sched.ntiles; t += nwarps) {
+      if (t < nchunks) {
+        const uint64_t v = (t << 5) + lane;
+        uint64_t b = 0;
+        uint32_t d = 0;
+        if (v < a.n) {
+          b = ldg(a.offs + v);
+          const uint64_t dd = ldg(a.offs + v + 1) - b;
+          d = dd > a.sched.heavy ? 0u : (uint32_t)dd;
+        }
+        if (!__any_sync(kFull, d != 0)) continue;
+        const float sum = chunk_row_sums(a.col, b, d, gather);
+        if (sum > 0.f) acc_cur[v] = sum;
+      } else {
+        const uint2 tv = a.sched.tiles[t - nchunks];
+        const uint64_t vb = ldg(a.offs + tv.x), ve = ldg(a.offs + tv.x + 1);
+        const uint64_t b = vb + (uint64_t)tv.y * a.sched.tile;
+        const float sum = tile_row_sum(a.col, b, min(ve, b + a.sched.tile), gather);
+        if (lane == 0 && sum > 0.f) atomicAdd(&acc_cur[tv.x], sum);
+      }
     }
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     const uint32_t accum = *reinterpret_cast<volatile uint32_t*>(&ctl->active[it % 3]);
@@ -805,12 +831,7 @@ __global__ void __launch_bounds__(kBlock) pr_pull_residual_persistent(PrArgs a) 
   }
 }
 
-// Pull-residual rounds over the binned layout (degree-ordered graphs): the
-// vertex pass of round it first closes round it - 1 (a positive sum becomes
-// the residual), then takes the residuals above tol (value += residual,
-// delta = residual * alpha / outdeg), and the gather sums the deltas over
-// the in-arcs.  The rounds, their deltas and the stopping rule are those of
-// pr_pull_residual_persistent; a round ends in two grid barriers, not three.
+// The same rounds over the binned layout (degree-ordered graphs).
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) pr_resid_binned(PrArgs a) {
   extern __shared__ float s_sum[];  // kBinPart floats
@@ -826,32 +847,7 @@ __global__ void __launch_bounds__(BLOCK, 1) pr_resid_binned(PrArgs a) {
       ctl->active[(it + 1) % 3] = 0;
       ctl->task_next[(it + 1) & 1] = 0u;
     }
-    uint32_t my_accum = 0;
-    for (uint64_t v = gtid; v < a.n; v += gthreads) {
-      float r = a.residual[v];
-      if (it > 0) {
-        const float sum = acc_prev[v];
-        if (sum > 0.f) r = sum;
-      }
-      // the sums of round it - 2, read by round it - 1: zeroed for this
-      // round's gather (zeroing the slots the last gather's atomics just
-      // updated stalls)
-      acc_cur[v] = 0.f;
-      float d = 0.f;
-      if (r > a.tol) {
-        a.value[v] += r;
-        const uint32_t k = a.nout[v];
-        if (k > 0) {
-          d = r * a.alpha / (float)k;
-          ++my_accum;
-        }
-        r = 0.f;
-      }
-      a.residual[v] = r;
-      a.delta[v] = d;
-    }
-    my_accum = __reduce_add_sync(kFull, my_accum);
-    if (lane_id() == 0 && my_accum) atomicAdd(&ctl->active[it % 3], my_accum);
+    resid_vertex_pass(a, it, acc_prev, acc_cur, gtid, gthreads);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     bin_gather<BLOCK>(a, a.delta, acc_cur, it, s_sum, &s_task);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
@@ -1334,7 +1330,7 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   if (kind == PrKind::Pull) {
     pr_pull_init<<<g->sm_count * 4, 256, 0, s>>>(a);
     a.zero_from = g->perm ? g->zero_from : n;
-    kfn = reinterpret_cast<const void*>(&pr_pull_persistent<kBlock, 2, 6>);
+    kfn = reinterpret_cast<const void*>(&pr_pull_persistent<kBlock, 6>);
     // the flat sweep needs the degree order: heavy rows first, the light rows' arcs one range
     if (g->perm && (g->order == GB_ORDER_DEGREE || g->order == GB_ORDER_DEGREE_UNSORTED)) {
       // degree-ordered: the binned layout (sequential streams, few
@@ -1363,6 +1359,7 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   } else if (kind == PrKind::PullResidual) {
     pr_resid_init<<<g->sm_count * 4, 256, 0, s>>>(a);
     GB_CUDA(cudaMemsetAsync(a.acc, 0, sizeof(float) * n, s));
+    GB_CUDA(cudaMemsetAsync(a.acc2, 0, sizeof(float) * n, s));
     kfn = reinterpret_cast<const void*>(&pr_pull_residual_persistent);
     if (g->perm && (g->order == GB_ORDER_DEGREE || g->order == GB_ORDER_DEGREE_UNSORTED)) {
       if (ensure_pr_bins(g, s) == GB_OK) {  // else the row sweep
@@ -1373,7 +1370,6 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
         a.b_rsrc = b->rsrc;
         a.b_tasks = b->tasks;
         a.b_ntasks = b->ntasks;
-        GB_CUDA(cudaMemsetAsync(a.acc2, 0, sizeof(float) * n, s));
         kfn = reinterpret_cast<const void*>(&pr_resid_binned<kBinBlock>);
         block = kBinBlock;
         smem = sizeof(float) * kBinPart;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from galois_b200 import DeviceGraph, GbError, erdos_renyi
+from galois_b200 import DeviceGraph, GbError, HostCSR, erdos_renyi
 from galois_b200 import _lib
 from galois_b200.graph import pack_graphs
 
@@ -45,8 +45,8 @@ def test_multigraph_matches_per_graph_oracle(cuda_device):
 def test_multigraph_labels_from_levels(cuda_device, sizes):
     """Labels taken from the BFS levels: graphs smaller than a warp's chunk, a
     source in the giant component, in a small one (the giant is unreached) and
-    without arcs; labels asked for alone take the other path."""
-    graphs = [erdos_renyi(n, 3.0, seed=i) for i, n in enumerate(sizes)]
+    without arcs."""
+    graphs = [erdos_renyi(n, 3.0, seed=i) if n > 1 else HostCSR(np.zeros(1), np.zeros(0)) for i, n in enumerate(sizes)]
     packed, first = pack_graphs(graphs)
     for pick in (np.argmax, np.argmin, lambda d: len(d) // 2):
         local = np.array([int(pick(g.degrees())) for g in graphs], np.uint32)
