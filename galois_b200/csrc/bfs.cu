@@ -28,6 +28,8 @@
 #include "device_graph.cuh"
 #include "frontier.cuh"
 
+#include <math_constants.h>
+
 #include <algorithm>
 
 namespace gb {
@@ -89,12 +91,84 @@ __global__ void bfs_init(BfsArgs a) {
   }
 }
 
-// Discovered vertices a warp collects before it looks at their degrees (one
-// step of 4 x 32 arcs always fits an empty stage).
+// Discovered vertices a warp collects in shared memory before it looks at
+// their degrees (one step of 4 x 32 arcs always fits an empty stage).
 constexpr uint32_t kStage = 128;
 
+// Queue a warp's n staged vertices: their degrees are read together, the light
+// ones go to light queue qb and the heavy ones' tiles to tile queue qb, both
+// reserved with one 64-bit atomic.  Adds the lane's share of the vertices and
+// of their degrees to items / deg.  `limit`: a degree sum above which nothing
+// is queued -- the next level then pulls, and reads the bitmap (the top hubs
+// of RMAT-20 have 40 K tiles, which one warp wrote and nobody read; a search
+// from one of them 191 -> 154 us).
+// All lanes call.
+__device__ __noinline__ void bfs_drain(const BfsArgs& a, const uint32_t* slots, uint32_t n, int qb,
+                                       FrontierCounters* c, double limit, uint32_t& items, unsigned long long& deg) {
+  constexpr int R = kStage / 32;
+  const uint32_t lane = lane_id();
+  __syncwarp();
+  uint32_t u[R], nt[R], tiles = 0, lights = 0;
+  uint64_t d[R];
+  unsigned lm[R];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const bool on = 32 * k + lane < n;
+    u[k] = on ? slots[32 * k + lane] : 0u;
+    d[k] = on ? ldg(a.offs + u[k] + 1) - ldg(a.offs + u[k]) : 0ull;
+    items += on ? 1u : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    deg += d[k];
+    nt[k] = d[k] > a.heavy ? (uint32_t)((d[k] + a.tile - 1) / a.tile) : 0u;
+    tiles += nt[k];
+    lm[k] = __ballot_sync(kFull, d[k] > 0 && d[k] <= a.heavy);
+    lights += __popc(lm[k]);
+  }
+  __syncwarp();  // the slots may be refilled
+  if ((double)warp_sum(deg) > limit) return;
+  uint32_t incl = tiles;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, incl, o);
+    if ((int)lane >= o) incl += t;
+  }
+  const uint32_t total = __shfl_sync(kFull, incl, 31);
+  unsigned long long base = 0;
+  if (lane == 0 && (lights | total))
+    base = atomicAdd(reinterpret_cast<unsigned long long*>(c), ((unsigned long long)total << 32) | lights);
+  base = __shfl_sync(kFull, base, 0);
+  uint32_t lpos = (uint32_t)base, tpos = (uint32_t)(base >> 32) + incl - tiles;
+  uint2* const tq = a.fq.tiles[qb];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    if ((lm[k] >> lane) & 1u) {
+      const uint32_t pos = lpos + __popc(lm[k] & ((1u << lane) - 1u));
+      if (pos < a.fq.light_cap) a.fq.light[qb][pos] = u[k];
+      else raise_err(&a.ctl->err, kDevOverflow);
+    }
+    lpos += __popc(lm[k]);
+    // a lane writes up to 8 tiles of its own, the warp the longer runs
+    uint32_t put = nt[k];
+    if ((uint64_t)tpos + put > a.fq.tile_cap) {
+      raise_err(&a.ctl->err, kDevOverflow);
+      put = tpos < a.fq.tile_cap ? a.fq.tile_cap - tpos : 0u;
+    }
+    if (put <= 8)
+      for (uint32_t i = 0; i < put; ++i) tq[tpos + i] = make_uint2(u[k], i);
+    for (unsigned big = __ballot_sync(kFull, put > 8); big; big &= big - 1) {
+      const int o = __ffs(big) - 1;
+      const uint32_t ov = __shfl_sync(kFull, u[k], o), on = __shfl_sync(kFull, put, o);
+      const uint32_t op = __shfl_sync(kFull, tpos, o);
+      for (uint32_t i = lane; i < on; i += 32) tq[op + i] = make_uint2(ov, i);
+    }
+    tpos += nt[k];
+  }
+}
+
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(BfsArgs a) {
+__global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(const __grid_constant__ BfsArgs a) {
   BfsCtl* ctl = a.ctl;
   const unsigned nblocks = gridDim.x;
   const uint64_t deadline = kernel_deadline();
@@ -115,6 +189,7 @@ __global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(BfsArgs a) {
   // and added to the global counters once per CTA
   __shared__ unsigned long long s_cnt[2];
   __shared__ uint32_t s_stage[BLOCK / 32][kStage];
+  uint32_t* const slots = s_stage[threadIdx.x >> 5];
   if (threadIdx.x == 0) s_cnt[0] = s_cnt[1] = 0;
   __syncthreads();
 
@@ -158,61 +233,40 @@ __global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(BfsArgs a) {
       // A pull level leaves only the frontier bitmap; a push level after it
       // first turns the bitmap into the queue.
       if (prev_pull) {
+        uint32_t n = 0, none = 0;
+        unsigned long long no_deg = 0;
         for (uint64_t base = gtid - lane; base < words; base += gthreads) {
           const uint64_t w = base + lane;
           uint32_t bits = w < words ? fb_rd[w] : 0u;
-          while (__any_sync(kFull, bits != 0)) {
-            const bool has = bits != 0;
-            const uint32_t v = has ? (uint32_t)(w << 5) + (uint32_t)(__ffs(bits) - 1) : 0u;
-            bits &= bits - 1;
-            push_discovered<false>(a.fq, L & 1, cur, has, v, a.offs, a.heavy, a.tile, &ctl->err);
+          for (unsigned m; (m = __ballot_sync(kFull, bits != 0)) != 0;) {
+            if (n + __popc(m) > kStage) {
+              bfs_drain(a, slots, n, L & 1, &cur, CUDART_INF, none, no_deg);
+              n = 0;
+            }
+            if (bits) {
+              slots[n + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(w << 5) + (uint32_t)(__ffs(bits) - 1);
+              bits &= bits - 1;
+            }
+            n += __popc(m);
           }
         }
+        if (n) bfs_drain(a, slots, n, L & 1, &cur, CUDART_INF, none, no_deg);
         if (!grid_barrier(&ctl->bar, nblocks, &ctl->err, deadline)) return;
       }
       const uint32_t q_light = min(cur.light, a.fq.light_cap);
       const uint32_t q_tiles = min(cur.tiles, a.fq.tile_cap);
-      uint32_t* const nq = a.fq.light[(L + 1) & 1];
       // Discovered vertices collect in shared memory, kStage per warp; their
       // degrees are read when the stage is full, all at once, not one
       // dependent read after every step that discovers something (directed
       // RMAT of 3 M vertices, 33 M arcs, push only: 481 -> 355 us with the
       // cheaper barrier; most steps discover something).
-      uint32_t* const slots = s_stage[threadIdx.x >> 5];
-      uint32_t staged = 0;
+      uint32_t staged = 0, q_items = 0;
+      unsigned long long q_deg = 0;
+      // the next level pulls when its degree sum is above this (the rule above)
+      const double limit = can_pull ? (double)edges_to_check / a.alpha : CUDART_INF;
       auto drain = [&]() {
-        constexpr int R = kStage / 32;
-        uint32_t u[R], base = 0, total = 0;
-        uint64_t d[R];
-        unsigned lm[R];
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-          const bool on = 32 * k + lane < staged;
-          u[k] = on ? slots[32 * k + lane] : 0u;
-          d[k] = on ? ldg(a.offs + u[k] + 1) - ldg(a.offs + u[k]) : 0ull;
-          my_items += on ? 1u : 0u;
-        }
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-          my_deg += d[k];
-          lm[k] = __ballot_sync(kFull, d[k] > 0 && d[k] <= a.heavy);
-          total += __popc(lm[k]);
-        }
-        if (lane == 0 && total) base = atomicAdd(&nxt.light, total);
-        base = __shfl_sync(kFull, base, 0);
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-          if ((lm[k] >> lane) & 1u) {
-            const uint32_t pos = base + __popc(lm[k] & ((1u << lane) - 1u));
-            if (pos < a.fq.light_cap) nq[pos] = u[k];
-            else raise_err(&ctl->err, kDevOverflow);
-          }
-          base += __popc(lm[k]);
-          warp_push_tiles(u[k], d[k] > a.heavy ? (uint32_t)((d[k] + a.tile - 1) / a.tile) : 0u,
-                          a.fq.tiles[(L + 1) & 1], &nxt.tiles, a.fq.tile_cap, &ctl->err);
-        }
+        bfs_drain(a, slots, staged, (L + 1) & 1, &nxt, limit, q_items, q_deg);
         staged = 0;
-        __syncwarp();
       };
       // Discovery over U steps at once: all lanes call with their candidates
       // (0xFFFFFFFF: none) and the visited words as loaded earlier (a stale
@@ -290,6 +344,8 @@ __global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(BfsArgs a) {
             }
           });
       if (staged) drain();
+      my_items = q_items;
+      my_deg = q_deg;
     } else {
       // Bottom-up over all vertices; warp-uniform trip count.  A warp owns
       // the 32 vertices of one bitmap word and is the only writer of that
