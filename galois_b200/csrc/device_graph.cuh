@@ -45,6 +45,8 @@ struct gb_graph {
   // PageRank pull on degree-ordered graphs: the binned layout of the arcs
   // (opaque, built and freed by pagerank.cu)
   struct PrBins* prb = nullptr;
+  // PageRank row sweeps in file order: the renamed columns (opaque, pagerank.cu)
+  struct PrHot* prh = nullptr;
   // bounded-degree graphs: the arcs as fixed-width rows (ell_d slots per
   // vertex, columns then uint32 weights, empty slots 0xFFFFFFFF), for SSSP
   uint32_t* ell = nullptr;
@@ -153,6 +155,8 @@ int ensure_transpose(gb_graph* g, cudaStream_t stream);
 void drop_derived(gb_graph* g);
 // Frees the PageRank binned layout (pagerank.cu).
 void free_pr_bins(gb_graph* g);
+// Frees the PageRank renamed columns (pagerank.cu).
+void free_pr_hot(gb_graph* g);
 
 // Relabelled graphs (reorder.cu).  result_buf returns the k-th n-word
 // staging buffer (k < 3).  finish_* map a result computed in internal ids

@@ -425,6 +425,7 @@ int gb_graph_free(gb_graph* g) {
   cudaFree(g->outdeg_of_stored);
   cudaFree(g->lr_rowid);
   gb::free_pr_bins(g);
+  gb::free_pr_hot(g);
   cudaFree(g->colsum);
   cudaFree(g->ell);
   if (g->ppr_free) g->ppr_free(g);

@@ -215,6 +215,7 @@ void drop_derived(gb_graph* g) {
   cudaFree(g->lr_rowid);
   g->lr_rowid = nullptr;
   free_pr_bins(g);
+  free_pr_hot(g);
   cudaFree(g->colsum);
   g->outdeg_of_stored = nullptr;
   g->colsum = nullptr;

@@ -433,6 +433,31 @@ def test_pagerank_binned_layout(cuda_device, case):
         assert abs(rst["iterations"] - rit) <= 2, case
 
 
+@pytest.mark.parametrize("n", [31, 49152, 49153, 70001])
+@pytest.mark.parametrize("order", [0, 1])
+def test_pagerank_row_sweep_edges(cuda_device, n, order):
+    """Row sweeps of graphs at and above the size from which file order renames
+    the columns (arcs leaning on a few vertices), the same in degree order;
+    rows of 0 to 9, 127-129 and 255-257 arcs and hubs of many tiles."""
+    rng = np.random.default_rng(n)
+    perm = rng.permutation(n)
+    deg = np.minimum(rng.zipf(1.6, n), 300)
+    deg[:16] = np.minimum([0, 1, 8, 9, 127, 128, 129, 255, 256, 257, 8192, 8193, 8449, 20000, 31, 33], n - 1)
+    src = np.repeat(perm, deg)
+    dst = perm[np.minimum((n * rng.random(len(src)) ** 8).astype(np.int64), n - 1)]
+    g = HostCSR.from_edges(n, src, dst)
+    want, it64 = oracle.pr_pull_topo_f64(g, 0.85, 1e-6, 1000)
+    rwant, rit = oracle.pr_pull_residual(g, 0.85, 1e-4, 1000, f64=True)
+    with DeviceGraph(g, symmetric=False, reorder=order) as dg:
+        for _ in range(2):
+            got, st = dg.pagerank_pull(0.85, 1e-6, 1000, stats=True)
+            assert np.max(np.abs(got.astype(np.float64) - want)) <= 1e-5  # the bound of the other pull tests
+            assert abs(st["iterations"] - it64) <= 2
+        rgot, rst = dg.pagerank_pull_residual(0.85, 1e-4, 1000, stats=True)
+        check_residual_parity(rgot, rwant, 1e-4, f"pull-residual n={n} order={order}")
+        assert abs(rst["iterations"] - rit) <= 2
+
+
 @pytest.mark.parametrize("method,kw", [("pagerank_pull_residual", {}), ("pagerank_push", {}),
                                        ("pagerank_push", {"algo": "async"})])
 def test_pagerank_residual_converges_to_fixed_point(cuda_device, method, kw):
