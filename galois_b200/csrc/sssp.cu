@@ -1675,13 +1675,21 @@ int run_sssp(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, gb_s
   const bool async = t.sssp_async > 0 && local_depth > 0 && g->max_degree <= t.heavy_degree &&
                      g->max_degree < 65536 && g->m < (1ull << 48);
   // regions in shared memory: asked for (sssp_async 3: whenever every
-  // region's arcs fit), or by default on a graph numbered by locality whose
-  // regions fit and keep at least 90 % of the arcs inside (measured on the
-  // 4096^2 grid: 29.3 ms against 38.5 ms for the phase-synchronous kernel)
+  // region's arcs fit), or by default on a bounded-degree graph, whatever its
+  // order, whose regions fit and keep most arcs inside: 90 % of them (measured
+  // on the 4096^2 grid by locality: 29.3 ms against 38.5 ms for the
+  // phase-synchronous kernel; file-order strips of a 1500 x 800 grid, 80 %:
+  // 13.0 against 9.2 ms), or half of them when every region has an SM of its
+  // own and none waits for another (file order, grids of 601 x 433, 89 %:
+  // 2.9 against 3.8 ms; 300 x 1000, 76 %: 4.9 / 5.2; 100 x 2000, 51 %: 8.6 /
+  // 9.2; 64 x 64: 0.12 / 0.38)
   bool region = false;
   const uint32_t nregions = (uint32_t)(((uint64_t)n + kRegion - 1) / kRegion);
-  if (t.sssp_async == 3 || (t.sssp_async == 0 && g->order == GB_ORDER_LOCALITY)) {
-    if (!g->region_arcs) {  // once per graph (and after a relabelling)
+  if (t.sssp_async == 3 || (t.sssp_async == 0 && (g->order == GB_ORDER_LOCALITY || local_depth > 0))) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    // a captured first call cannot wait for the count: it runs as if it failed
+    if (!g->region_arcs) GB_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (!g->region_arcs && cap == cudaStreamCaptureStatusNone) {  // once per graph (and after a relabelling)
       int rst = ws_reserve(g, 256, s);
       if (rst != GB_OK) return rst;
       unsigned long long* dout = static_cast<unsigned long long*>(g->ws);
@@ -1694,8 +1702,9 @@ int run_sssp(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, gb_s
       g->region_arcs = hout[0] + 1;
       g->region_local = g->m ? (double)hout[1] / (double)g->m : 1.0;
     }
-    const bool fits = g->region_arcs - 1 <= kRegionArcs;
-    region = t.sssp_async == 3 ? fits : fits && g->region_local >= 0.9;
+    const bool fits = g->region_arcs && g->region_arcs - 1 <= kRegionArcs;
+    const double keep = nregions <= (uint32_t)g->sm_count ? 0.5 : 0.9;
+    region = t.sssp_async == 3 ? fits : fits && g->region_local >= keep;
   }
   if (region) return run_sssp_region(g, src, shift, nregions, dist_out, out_dev, stats, s);
   FrontierLayout fl = frontier_layout(n, g->m, t.heavy_degree, t.tile_edges);

@@ -262,9 +262,11 @@ typedef struct gb_tuning {
                             GB_ORDER_LOCALITY; otherwise as 1); stats:
                             rounds = region visits, pull_rounds =
                             shared-memory rounds;
-                            0 = library default: regions on a
-                            GB_ORDER_LOCALITY graph whose regions fit and
-                            keep >= 90 % of the arcs inside, else a grid
+                            0 = library default: regions on a graph of
+                            low degree (local queues on, or
+                            GB_ORDER_LOCALITY) whose regions fit and keep
+                            >= 90 % of the arcs inside (>= 50 % when there
+                            is an SM for every region), else a grid
                             barrier after every phase; < 0 = a grid
                             barrier after every phase */
 } gb_tuning;

@@ -245,3 +245,22 @@ def test_auto_order_and_default_region_kernel(cuda_device):
                 got, st = dg.sssp(src, shift, stats=True)
                 assert (got == want).all() and st["pull_rounds"] == 0, (src, shift)
                 dg.set_tuning(sssp_async=0)
+
+
+@pytest.mark.parametrize("rows,cols,shuffled", [(1, 2047, False), (1, 2048, False), (33, 65, False), (90, 433, False),
+                                                (601, 433, False), (100, 2900, False), (90, 433, True)])
+def test_default_region_rule_in_file_order(cuda_device, rows, cols, shuffled):
+    """A grid in file order takes the region kernel when its regions of 2048
+    ids keep at least half of the arcs and each has an SM; with its ids
+    shuffled it does not.  Same distances either way, from the first vertex,
+    the middle and the last."""
+    g = grid2d(rows, cols)
+    if shuffled:
+        perm = np.random.default_rng(1).permutation(g.n)
+        g = HostCSR.from_edges(g.n, perm[np.repeat(np.arange(g.n), g.degrees())], perm[g.col])
+    assign_weights_u32(g, 1, 255, seed=rows)
+    with DeviceGraph(g, symmetric=True) as dg:
+        for src in (0, g.n // 2, g.n - 1):
+            got, st = dg.sssp(src, 13, stats=True)
+            assert (got == oracle.sssp_dijkstra(g, src)).all()
+            assert (st["pull_rounds"] > 0) == (not shuffled)
