@@ -16,7 +16,7 @@
 // read once per iteration for all B columns.  With fewer columns a row takes
 // fewer lanes (B / 4, rounded up to a power of two) and the warp takes that
 // many more arcs at once.  A warp takes the rows of a task one after another,
-// the next row's column ids and weights already loaded, eight 512-byte rows in
+// the next row's column ids and weights already loaded, four 512-byte rows in
 // flight; rows above the tile size are split into tiles whose partial rows
 // are stored and then summed in arc order (the same result every time).  The forward pulls over the in-arcs of
 // the device transpose, the adjoint over the out-arcs of the CSR; a row
@@ -27,7 +27,11 @@
 // RMAT-20, B = 128 (82 forward and 91 adjoint iterations): with tasks of up to
 // 1024 arcs, four rows in flight and no loads ahead of the row, forward plus
 // adjoint took 270 ms (a third of the warps' time waiting at the barriers);
-// this takes 193 ms, 1.07 ms an iteration or 7.6 TB/s of gathered rows.
+// the walk above 187 ms, with more CTAs and fewer rows in flight each 173 ms,
+// 1.0 ms an iteration or 8.2 TB/s of gathered rows (iterate_kernel below).
+// 512-byte rows taken as 128- or 256-byte slices, a pass over the rows for
+// each, hit L1 more often and still took 295 and 208 ms: the work per row is
+// paid once for each slice.
 
 #include <algorithm>
 #include <vector>
@@ -187,8 +191,8 @@ __device__ __forceinline__ ArcLoad load_arcs(const uint32_t* __restrict__ col, c
 }
 
 // Rows of B floats handled by LPA lanes (4 columns each), G = 32 / LPA arcs
-// per step, U steps in flight: 8 rows of 512 bytes at B = 128, at least two
-// steps at small B.
+// per step; U steps in flight in the gradient (8 rows of 512 bytes at B = 128,
+// at least two steps at small B; the iteration takes its own).
 template <int LPA>
 struct Wide {
   static constexpr int G = 32 / LPA;
@@ -197,10 +201,10 @@ struct Wide {
 
 // Sum over arcs [b, e) of wn * x[col] for this lane's 4 columns; `first` holds
 // the row's first 32 arcs.  Every group of LPA lanes returns the whole sum.
-template <int LPA>
+template <int LPA, int U>
 __device__ __forceinline__ float4 row_sum(const IterArgs& a, const float* __restrict__ x, uint64_t b, uint64_t e,
                                           ArcLoad m) {
-  constexpr int G = Wide<LPA>::G, U = Wide<LPA>::U;
+  constexpr int G = Wide<LPA>::G;
   const uint32_t lane = lane_id(), sub = lane % LPA, grp = lane / LPA;
   const bool act = 4 * sub < a.B;
   const float* __restrict__ xs = x + 4 * sub;
@@ -279,8 +283,8 @@ __device__ __forceinline__ uint32_t ppr_rows_per_task(uint32_t n, uint64_t nwarp
 }
 
 // LPA: lanes per row of B floats; 0 for B = 1 (lanes over arcs).
-template <int LPA>
-__global__ void __launch_bounds__(kPprBlock, LPA ? 3 : 4) ppr_iterate(IterArgs a) {
+template <int LPA, int U, int MINB>
+__global__ void __launch_bounds__(kPprBlock, MINB) ppr_iterate(IterArgs a) {
   constexpr bool WIDE = LPA != 0;
   constexpr int L = WIDE ? LPA : 1;
   __shared__ __align__(16) float s_diff[kPprWarps][128];  // written as float4
@@ -331,7 +335,7 @@ __global__ void __launch_bounds__(kPprBlock, LPA ? 3 : 4) ppr_iterate(IterArgs a
         const uint64_t b = vb + (uint64_t)tv.y * tile, e = min(ve, b + tile);
         float* h = a.part + t * a.B;
         if constexpr (WIDE) {
-          const float4 acc = row_sum<L>(a, x, b, e, load_arcs(a.col, a.wn, b, e));
+          const float4 acc = row_sum<L, U>(a, x, b, e, load_arcs(a.col, a.wn, b, e));
           if (act) reinterpret_cast<float4*>(h)[lane] = acc;
         } else {
           float s = 0.f;
@@ -343,7 +347,7 @@ __global__ void __launch_bounds__(kPprBlock, LPA ? 3 : 4) ppr_iterate(IterArgs a
         ppr_rows(a.offs, a.col, a.wn, a.n, (t - a.sched.ntiles) * rpt, rpt, tile,
                  [&](uint32_t r, uint64_t b, uint64_t e, ArcLoad m) {
                    const float4 o = old_row(r);  // in flight beside the gathers
-                   finish(r, row_sum<L>(a, x, b, e, m), o);
+                   finish(r, row_sum<L, U>(a, x, b, e, m), o);
                  });
       } else {
         // 32 rows' arcs walked together, four steps of loads in flight; a
@@ -515,15 +519,30 @@ int lanes_per_row(uint32_t B) {
   return l;
 }
 
-const void* iterate_kernel(uint32_t B) {
+template <int LPA, int U, int MINB>
+const void* iterate_ptr() {
+  return reinterpret_cast<const void*>(&ppr_iterate<LPA, U, MINB>);
+}
+
+// Gathers in flight per warp against warps on the SM: four CTAs of 256 threads
+// leave 64 registers, enough for four steps in flight (two for rows of at most
+// 64 bytes), and hide more than three CTAs with twice the steps.  Forward +
+// adjoint, edge factor 16, three CTAs / four, ms: RMAT-20 B = 128 187 / 173,
+// 64 127 / 108, 32 106 / 76, 12 72 / 61, 8 57 / 51, 4 51 / 44; 30 K vertices
+// B = 128 7.5 / 7.05, 32 3.95 / 3.6, 12 5.1 / 4.6.  At
+// 16 lanes per row nothing is gained while the iterate fits L2 (B = 64, 200 K
+// vertices 25.3 / 26.7, 90 K 9.8 / 10.0), and three CTAs stay.
+constexpr uint64_t kL2Iterate = 126ull << 20;
+
+const void* iterate_kernel(uint32_t B, uint32_t n) {
   switch (lanes_per_row(B)) {
-    case 0: return reinterpret_cast<const void*>(&ppr_iterate<0>);
-    case 1: return reinterpret_cast<const void*>(&ppr_iterate<1>);
-    case 2: return reinterpret_cast<const void*>(&ppr_iterate<2>);
-    case 4: return reinterpret_cast<const void*>(&ppr_iterate<4>);
-    case 8: return reinterpret_cast<const void*>(&ppr_iterate<8>);
-    case 16: return reinterpret_cast<const void*>(&ppr_iterate<16>);
-    default: return reinterpret_cast<const void*>(&ppr_iterate<32>);
+    case 0: return iterate_ptr<0, 2, 4>();
+    case 1: return iterate_ptr<1, 2, 4>();
+    case 2: return iterate_ptr<2, 2, 4>();
+    case 4: return iterate_ptr<4, 2, 4>();
+    case 8: return iterate_ptr<8, 4, 4>();
+    case 16: return sizeof(float) * B * (uint64_t)n > kL2Iterate ? iterate_ptr<16, 4, 4>() : iterate_ptr<16, 4, 3>();
+    default: return iterate_ptr<32, 4, 4>();
   }
 }
 
@@ -637,7 +656,7 @@ int solve(gb_graph* g, PprState* st, bool adjoint, uint32_t B, const float* src,
   GB_CUDA(cudaMemsetAsync(st->flags, 0, sizeof(uint32_t) * ((g->n + 31) / 32), s));
   ppr_seed<<<g->sm_count * 8, 256, 0, s>>>(src, scale, g->n, B, st->flags, out, tmp, st->l1 + 3 * 128);  // x0 = scale * src
   GB_CUDA(cudaGetLastError());
-  const void* kfn = iterate_kernel(B);
+  const void* kfn = iterate_kernel(B, g->n);
   int grid = coop_grid(g, kfn, kPprBlock, 0, 0);
   // no more CTAs than there is work for: every CTA takes part in the barriers
   const uint64_t work = a.sched.ntiles + (B > 1 ? (uint64_t)g->n : ((uint64_t)g->n + 31) / 32);
