@@ -63,15 +63,14 @@ struct PrBins {
 // The row sweeps' renamed columns of a graph in file order (ensure_hot), cached
 // in the graph handle.
 struct PrHot {
-  uint32_t* rank = nullptr;  // [n] vertex -> slot of its contribution (nullptr: not renamed)
-  uint32_t* col = nullptr;   // [m] the columns as slots
+  uint32_t* col = nullptr;   // [m] the columns as slots, then rank (nullptr: not renamed)
+  uint32_t* rank = nullptr;  // [n] vertex -> slot of its contribution
 };
 
 namespace gb {
 
 void free_pr_hot(gb_graph* g) {
   if (!g->prh) return;
-  cudaFree(g->prh->rank);
   cudaFree(g->prh->col);
   delete g->prh;
   g->prh = nullptr;
@@ -1152,30 +1151,42 @@ __global__ void hot_col_kernel(const uint32_t* __restrict__ col, uint64_t m, con
 // Where it pays: the contributions do not fit L1 anyway (n > kHotSlots), and
 // the kHotSlots most gathered vertices (192 KB) take a quarter of the arcs
 // (RMAT-21 directed: 67 %; a uniform graph or a grid: kHotSlots / n).
-// A graph that does not qualify, or whose copy cannot be allocated, keeps its
-// columns.  Pull-residual: RMAT-21 directed (34 rounds) 5.98 -> 5.39 ms,
+// A graph that does not qualify keeps its columns; so does one whose copy
+// would take more than a quarter of the free memory, and one whose first call
+// is being captured into a graph (the choice waits for a count).
+// Pull-residual: RMAT-21 directed (34 rounds) 5.98 -> 5.39 ms,
 // RMAT-22 symmetric 23.7 -> 16.9 ms (first call 25.2 -> 20.0); pull-topological
 // on the latter 12.4 -> 10.6 ms (13.8 -> 13.6).
 constexpr uint32_t kHotSlots = 49152;
 constexpr double kHotShare = 0.25;
 
-int ensure_hot(gb_graph* g, cudaStream_t s) {
-  if (g->prh) return GB_OK;
+// Workspace of ensure_hot, which runs before the solve carves its own from the
+// same block (0: nothing to do).
+int hot_scratch(gb_graph* g, cudaStream_t s, size_t* bytes, size_t* sort_bytes) {
+  *bytes = 0;
+  if (g->prh || g->m == 0 || g->n <= kHotSlots) return GB_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  GB_CUDA(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return GB_OK;
+  size_t free_bytes = 0, total_bytes = 0;
+  GB_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (sizeof(uint32_t) * (g->m + g->n) > free_bytes / 4) return GB_OK;
+  cub::DoubleBuffer<uint32_t> key(nullptr, nullptr), id(nullptr, nullptr);
+  GB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, *sort_bytes, key, id, (int64_t)g->n, 0, 32, s));
+  *bytes = carve_size<unsigned long long>(1) + 4 * carve_size<uint32_t>(g->n) + carve_size<char>(*sort_bytes);
+  return GB_OK;
+}
+
+int ensure_hot(gb_graph* g, size_t sort_bytes, cudaStream_t s) {
   const uint32_t n = g->n;
   const uint64_t m = g->m;
   PrHot* h = new (std::nothrow) PrHot;
   if (!h) GB_FAIL(GB_ERR_OOM, "pagerank: host allocation failed");
   g->prh = h;
-  if (m == 0 || n <= kHotSlots) return GB_OK;
-  size_t sort_bytes = 0;
-  cub::DoubleBuffer<uint32_t> key(nullptr, nullptr), id(nullptr, nullptr);
-  GB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, key, id, (int64_t)n, 0, 32, s));
-  const size_t need = carve_size<unsigned long long>(1) + 4 * carve_size<uint32_t>(n) + carve_size<char>(sort_bytes);
-  int st = ws_reserve(g, need, s);
-  if (st != GB_OK) return st;
   Carver cv(g->ws);
   unsigned long long* arcs = cv.take<unsigned long long>(1);
   unsigned long long* harcs = static_cast<unsigned long long*>(g->pinned);
+  cub::DoubleBuffer<uint32_t> key(nullptr, nullptr), id(nullptr, nullptr);
   for (int k = 0; k < 2; ++k) {
     key.d_buffers[k] = cv.take<uint32_t>(n);
     id.d_buffers[k] = cv.take<uint32_t>(n);
@@ -1189,13 +1200,12 @@ int ensure_hot(gb_graph* g, cudaStream_t s) {
   GB_CUDA(cudaMemcpyAsync(harcs, arcs, sizeof(*arcs), cudaMemcpyDeviceToHost, s));
   GB_CUDA(cudaStreamSynchronize(s));
   if ((double)*harcs < kHotShare * (double)m) return GB_OK;
-  if (cudaMalloc(&h->rank, sizeof(uint32_t) * n) != cudaSuccess ||
-      cudaMalloc(&h->col, sizeof(uint32_t) * m) != cudaSuccess) {
+  if (cudaMalloc(&h->col, sizeof(uint32_t) * (m + n)) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(h->rank);
-    h->rank = nullptr;
+    h->col = nullptr;
     return GB_OK;
   }
+  h->rank = h->col + m;
   hot_rank_kernel<<<grid, 256, 0, s>>>(id.Current(), n, h->rank);
   hot_col_kernel<<<grid, 256, 0, s>>>(g->col, m, h->rank, h->col);
   GB_CUDA(cudaGetLastError());
@@ -1393,10 +1403,6 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
     if (st != GB_OK) return st;
     st = ensure_nout(g, s);
     if (st != GB_OK) return st;
-    if (!g->perm) {
-      st = ensure_hot(g, s);
-      if (st != GB_OK) return st;
-    }
   }
   FrontierLayout fl = frontier_layout(n, g->m, t.heavy_degree, t.tile_edges);
   // Async: the initial worklist (every vertex, 32 per chunk) plus room for
@@ -1407,8 +1413,23 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   if (kind != PrKind::Pull) need += 2 * carve_size<float>(n);
   if (kind == PrKind::Push) need += 3 * carve_size<uint32_t>(n) + fl.bytes;
   if (kind == PrKind::PushAsync) need += carve_size<char>(worklists::ring_bytes(cap));
-  st = ws_reserve(g, need, s);
+  const bool rows = (kind == PrKind::Pull || kind == PrKind::PullResidual) && !g->perm;  // row sweeps in file order
+  size_t hot = 0, sort_bytes = 0;
+  if (rows) {
+    st = hot_scratch(g, s, &hot, &sort_bytes);
+    if (st != GB_OK) return st;
+  }
+  st = ws_reserve(g, std::max(need, hot), s);
+  if (st != GB_OK && hot > need) {
+    clear_error();
+    hot = 0;
+    st = ws_reserve(g, need, s);
+  }
   if (st != GB_OK) return st;
+  if (hot) {
+    st = ensure_hot(g, sort_bytes, s);
+    if (st != GB_OK) return st;
+  }
   Carver cv(g->ws);
   PrArgs a{};
   a.ctl = cv.take<PrCtl>(1);
@@ -1441,7 +1462,7 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   a.sched = sched;
   a.heavy = t.heavy_degree;
   a.tile = t.tile_edges;
-  if ((kind == PrKind::Pull || kind == PrKind::PullResidual) && !g->perm && g->prh->col) {
+  if (rows && g->prh && g->prh->col) {
     a.rank = g->prh->rank;
     a.col = g->prh->col;
   }
