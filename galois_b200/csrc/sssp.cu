@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(BLOCK) sssp_persistent(SsspArgs a) {
       const uint64_t est = bm_in ? 16ull * bm_count : 16ull * q_light + (uint64_t)a.tile * q_tiles;
       const bool bm_out = kBitmap && est > a.bm_min;
       uint32_t* const act_next = a.act[(P + 1) % 3];
-      uint32_t my_push = 0;  // lane 0: this warp's bit-setting reductions
+      uint32_t my_push = 0;  // this lane's bit-setting reductions
       uint32_t lq_n = 0;  // warp-uniform local queue length
       WarpStage<kStage> stage{s_stage[threadIdx.x >> 5], 0u};
       uint32_t* const nq = a.fq.light[qnext];
@@ -248,31 +248,31 @@ __global__ void __launch_bounds__(BLOCK) sssp_persistent(SsspArgs a) {
         warp_push(far, u, farq, &ctl->far_count[fp], a.n, &ctl->err);
       };
       const bool need_deg = !a.all_light || a.local_depth > 0;
+      // bitmap output: no reply awaited.  The bit marks u for the next phase,
+      // which reads dist[u] when it expands u (a bit set by a candidate that
+      // lost to a smaller one only costs that re-expansion).
+      auto mark = [&](bool valid, uint32_t u, uint32_t nd, uint32_t du) {
+        bool far = false;
+        if (valid && nd < du) {
+          red_min_u32(&a.dist[u], nd);
+          const uint32_t bit = 1u << (u & 31);
+          if (nd < hi) {
+            red_or_u32(&act_next[u >> 5], bit);
+            ++my_push;
+            ++my_relax;
+          } else if (!(a.infar[u >> 5] & bit)) {
+            far = !(atomicOr(&a.infar[u >> 5], bit) & bit);
+            my_relax += far;
+          }
+        }
+        if (__any_sync(kFull, far)) warp_push(far, u, farq, &ctl->far_count[fp], a.n, &ctl->err);
+      };
       // du: dist[u] as loaded with the arc, or ~0 to skip the pre-check (a
       // stale value only costs an extra atomic; the atomicMin decides)
       auto relax = [&](bool valid, uint32_t u, uint32_t nd, uint32_t du) {
         bool near = false, far = false;
         if (bm_out) {
-          // no reply awaited: the bit marks u for the next phase, which reads
-          // dist[u] when it expands u (a bit set by a candidate that lost to
-          // a smaller one only costs that re-expansion)
-          if (valid && nd < du) {
-            red_min_u32(&a.dist[u], nd);
-            const uint32_t bit = 1u << (u & 31);
-            if (nd < hi) {
-              red_or_u32(&act_next[u >> 5], bit);
-              near = true;
-            } else if (!(a.infar[u >> 5] & bit)) {
-              far = !(atomicOr(&a.infar[u >> 5], bit) & bit);
-            }
-          }
-          const unsigned nm = __ballot_sync(kFull, near);
-          const unsigned rm = __ballot_sync(kFull, near || far);
-          if (lane == 0) {
-            my_push += __popc(nm);
-            my_relax += __popc(rm);
-          }
-          if (__any_sync(kFull, far)) warp_push(far, u, farq, &ctl->far_count[fp], a.n, &ctl->err);
+          mark(valid, u, nd, du);
           return;
         }
         uint64_t ub = 0, deg = 1;
@@ -344,7 +344,105 @@ __global__ void __launch_bounds__(BLOCK) sssp_persistent(SsspArgs a) {
           for (int k = 0; k < U; ++k) relax(valid[k], u[k], nd[k], du[k]);
         }
       };
-      if (kBitmap && bm_in) {
+      if (kBitmap && bm_in && bm_out) {
+        // bitmap to bitmap, where most arcs of a power-law graph are relaxed:
+        // the words as below, two non-zero ones together, their light vertices
+        // gathered in the local queue (unused otherwise without local rounds)
+        // and expanded 32 at a time.  A phase is bound by the loads that a
+        // warp waits for in turn: a word's rows, columns and distances one
+        // word after another, and a tile's offsets, then 128 arcs at a time.
+        // RMAT-22 directed (11 phases, 2.3 m arcs) 1165 -> 937 us, 4 M
+        // vertices of edge factor 4 766 -> 542, 30 K 233 -> 196.  (Expanding
+        // only the nearest quarter of the arcs each phase relaxes 1.6 m in 15
+        // phases and takes longer; eight lanes per row do too.)
+        const uint32_t* act = a.act[P % 3];
+        uint32_t held = 0;
+        auto drain = [&](uint32_t take) {
+          held -= take;
+          const uint4 ent = lane < take ? lq[held + lane] : make_uint4(0u, 0u, 0u, 0u);
+          __syncwarp();
+          my_scanned += ent.z;
+          warp_expand_mlp<4, uint2>(
+              ((uint64_t)ent.y << 32) | ent.x, ent.z, ent.w,
+              [&](bool valid, uint64_t e, uint32_t) { return valid ? ldg(a.col + e) : 0u; },
+              [&](bool valid, uint64_t e, uint32_t u, uint32_t dsrc) {
+                return valid ? make_uint2(dsrc + ldg(a.w + e), a.dist[u]) : make_uint2(0u, 0u);
+              },
+              [&](bool valid, uint32_t, uint32_t, uint32_t u, uint2 v2) { mark(valid, u, v2.x, v2.y); });
+        };
+        for (uint64_t base = gwarp; base < words; base += nwarps << 5) {
+          const uint64_t wi = base + (uint64_t)lane * nwarps;
+          const uint32_t word = wi < words ? __ldcg(act + wi) : 0u;
+          unsigned nz = __ballot_sync(kFull, word != 0u);
+          while (nz) {
+            constexpr int U = 2;
+            uint64_t b[U];
+            uint32_t d[U], dv[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+              const int j = nz ? __ffs(nz) - 1 : 0;
+              const uint32_t bits = nz ? __shfl_sync(kFull, word, j) : 0u;
+              nz &= nz - 1u;
+              b[k] = 0;
+              d[k] = dv[k] = 0;
+              if ((bits >> lane) & 1u) {
+                const uint64_t v = ((base + (uint64_t)j * nwarps) << 5) + lane;  // < n when its bit is set
+                b[k] = ldg(a.offs + v);
+                const uint64_t dd = ldg(a.offs + v + 1) - b[k];
+                d[k] = dd <= a.heavy ? (uint32_t)dd : 0u;
+                dv[k] = __ldcg(a.dist + v);
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+              const unsigned tm = __ballot_sync(kFull, d[k] != 0);
+              if (d[k])
+                lq[held + __popc(tm & lanemask_lt)] = make_uint4((uint32_t)b[k], (uint32_t)(b[k] >> 32), d[k], dv[k]);
+              __syncwarp();
+              held += __popc(tm);
+              if (held >= 32) drain(32);
+            }
+          }
+        }
+        if (held) drain(held);
+        // heavy vertices: the cached tile schedule, strided the same way, 256
+        // arcs a step: columns and the vertex's distance, then weights and
+        // the targets' distances
+        for (uint64_t t0 = gwarp; t0 < a.sw_ntiles; t0 += nwarps << 5) {
+          const uint64_t ti = t0 + (uint64_t)lane * nwarps;
+          uint32_t tv = 0, td = 0;
+          uint64_t tb = 0;
+          if (ti < a.sw_ntiles) {
+            const uint2 t = a.sw_tiles[ti];
+            tv = t.x;
+            if ((__ldcg(act + (tv >> 5)) >> (tv & 31)) & 1u) {
+              const uint64_t vb = ldg(a.offs + tv), ve = ldg(a.offs + tv + 1);
+              tb = vb + (uint64_t)t.y * a.tile;
+              td = (uint32_t)(min(ve, tb + a.tile) - tb);
+            }
+          }
+          my_scanned += td;
+          for (unsigned m = __ballot_sync(kFull, td != 0); m; m &= m - 1u) {
+            const int j = __ffs(m) - 1;
+            const uint64_t b = __shfl_sync(kFull, tb, j);
+            const uint32_t d = __shfl_sync(kFull, td, j);
+            const uint32_t dsrc = __ldcg(a.dist + __shfl_sync(kFull, tv, j));
+            constexpr int U = 8;
+            for (uint32_t i0 = lane; i0 < d + lane; i0 += 32 * U) {
+              uint32_t u[U], w[U], du[U];
+#pragma unroll
+              for (int k = 0; k < U; ++k) u[k] = i0 + 32 * k < d ? ldg(a.col + b + i0 + 32 * k) : 0xFFFFFFFFu;
+#pragma unroll
+              for (int k = 0; k < U; ++k) {
+                w[k] = u[k] != 0xFFFFFFFFu ? ldg(a.w + b + i0 + 32 * k) : 0u;
+                du[k] = u[k] != 0xFFFFFFFFu ? a.dist[u[k]] : 0u;
+              }
+#pragma unroll
+              for (int k = 0; k < U; ++k) mark(u[k] != 0xFFFFFFFFu, u[k], dsrc + w[k], du[k]);
+            }
+          }
+        }
+      } else if (kBitmap && bm_in) {
         // bitmap frontier: a warp owns words gwarp, gwarp + nwarps, ... (32
         // ids each; strided so that the dense low ids of a degree-ordered
         // graph spread over all warps), loads 32 of them per step and expands
@@ -444,6 +542,7 @@ __global__ void __launch_bounds__(BLOCK) sssp_persistent(SsspArgs a) {
       }
       stage.flush(nq, &nxt.light, a.fq.light_cap, &ctl->err);
       if (bm_out) {  // grid-uniform branch: the CTA's bit-setting reductions, added once
+        my_push = __reduce_add_sync(kFull, my_push);
         if (lane == 0 && my_push) atomicAdd_block(&s_push, my_push);
         __syncthreads();
         if (threadIdx.x == 0) {

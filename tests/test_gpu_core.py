@@ -433,6 +433,29 @@ def test_pagerank_binned_layout(cuda_device, case):
         assert abs(rst["iterations"] - rit) <= 2, case
 
 
+@pytest.mark.parametrize("n", [4097, 20000])
+@pytest.mark.parametrize("shift,tile,order", [(13, 0, 0), (13, 96, 1), (13, 512, 0), (7, 0, 1), (5, 256, 0)])
+def test_sssp_bitmap_phases(cuda_device, n, shift, tile, order):
+    """Bitmap phases over rows of 0, 1 and up to a warp's steps and tiles'
+    edges (128/129 arcs: light/heavy; 255-257, 512/513: tiles), hubs of many
+    tiles, words with one and with all 32 vertices active; with small deltas
+    also the far pile.  Exact against Dijkstra, twice."""
+    rng = np.random.default_rng(n + shift)
+    deg = np.where(rng.random(n) < 0.6, rng.integers(0, 8, n), rng.integers(0, 140, n))
+    deg[64:128] = 0
+    deg[:16] = np.minimum([0, 1, 31, 32, 33, 127, 128, 129, 255, 256, 257, 511, 512, 513, 3000, 4000], n - 1)
+    src = np.repeat(rng.permutation(n), deg)
+    g = HostCSR.from_edges(n, src, rng.integers(0, n, len(src)))
+    assign_weights_u32(g, 1, 255, seed=3)
+    with DeviceGraph(g, symmetric=False, reorder=order) as dg:
+        if tile:
+            dg.set_tuning(tile_edges=tile)
+        for s in (int(np.argmax(g.degrees())), int(np.flatnonzero(g.degrees())[-1])):
+            want = oracle.sssp_dijkstra(g, s)
+            for _ in range(2):
+                assert (dg.sssp(s, shift) == want).all()
+
+
 @pytest.mark.parametrize("n", [31, 49152, 49153, 70001])
 @pytest.mark.parametrize("order", [0, 1])
 def test_pagerank_row_sweep_edges(cuda_device, n, order):
