@@ -48,16 +48,15 @@
 #include <cstring>
 
 // The binned layout of a degree-ordered graph's arcs for the PageRank pull
-// (pr_pull_binned): one device allocation, cached in the graph handle.
+// (pr_pull_binned), cached in the graph handle.
 struct PrBins {
-  void* mem = nullptr;
-  uint16_t* dst = nullptr;
-  uint8_t* roff = nullptr;
+  void* mem = nullptr;       // the arrays but rdst
+  uint16_t* src = nullptr;
+  uint8_t* flag = nullptr;
   uint32_t* crun = nullptr;
-  uint32_t* rsrc = nullptr;  // per run: its source
+  uint32_t* rdst = nullptr;  // per run: its destination
   uint4* tasks = nullptr;
   uint32_t ntasks = 0;
-  uint64_t npairs = 0, nchunks = 0;
 };
 
 // The row sweeps' renamed columns of a graph in file order (ensure_hot), cached
@@ -79,6 +78,7 @@ void free_pr_hot(gb_graph* g) {
 void free_pr_bins(gb_graph* g) {
   if (!g->prb) return;
   cudaFree(g->prb->mem);
+  cudaFree(g->prb->rdst);
   delete g->prb;
   g->prb = nullptr;
 }
@@ -140,11 +140,13 @@ struct PrArgs {
   const uint8_t* __restrict__ lr_rowd;
   uint64_t lr_arc0, lr_arc1;
   // binned pull (degree-ordered graphs, pr_pull_binned)
-  const uint16_t* __restrict__ b_dst;   // per padded arc: destination - partition base (0xFFFF: padding)
-  const uint8_t* __restrict__ b_roff;   // per padded arc: its run - the chunk's first run
-  const uint32_t* __restrict__ b_crun;  // per 256-arc chunk: its first run
-  const uint32_t* __restrict__ b_rsrc;  // per run: its source
-  const uint4* __restrict__ b_tasks;    // (partition base, vertices | multi << 31, chunk begin, chunk end)
+  const uint16_t* __restrict__ b_src;   // per padded arc: source - block base (kBinPart: padding)
+  const uint8_t* __restrict__ b_flag;   // per 8 arcs: which of them start a run
+  const uint32_t* __restrict__ b_crun;  // per 256-arc chunk: its first run; then the number of runs
+  const uint32_t* __restrict__ b_rdst;  // per run: its destination
+  double* hacc;       // binned: sums of the top rows (ids below b_nheavy), [2][b_nheavy], in acc's place
+  uint32_t b_nheavy;  // (0: not binned)
+  const uint4* __restrict__ b_tasks;    // (block base, sources, chunk begin, chunk end)
   uint32_t b_ntasks;
   const uint32_t* __restrict__ rank;  // row sweeps: slot of a vertex's contribution (nullptr: its id)
 };
@@ -487,151 +489,202 @@ __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_flat(PrArgs a) {
 }
 
 // ---- binned pull (degree-ordered graphs) --------------------------------------
-// The destinations are cut into partitions of kBinPart consecutive ids, few
-// enough that a partition's sums fit in shared memory.  Inside a partition
-// the in-arcs are ordered by source, so the arcs from one source form a run;
-// the arcs are stored in 256-arc chunks (per arc a 2-byte local destination
-// and a 1-byte offset of its run from the chunk's first run, the chunk's arcs
-// sorted by destination), and per run its source.  Per iteration
-//   gather: a CTA takes a task (a range of chunks of one partition), streams
-//     the chunks, reads each run's source and that source's contribution
-//     (the contributions, 4 bytes per vertex, stay mostly in L2), sums equal
-//     destinations of a lane's 8 arcs in registers and adds them into the
-//     partition's sums in shared memory, then writes the sums out (added
-//     with atomics when the partition has several tasks);
+// The sources are cut into blocks of kBinPart consecutive ids whose
+// contributions fit in shared memory.  The in-arcs of a block are ordered by
+// destination, so the arcs into one destination form a run; they are stored in
+// 256-arc chunks (per arc a 2-byte local source, per 8 arcs a byte that says
+// which start a run; every chunk starts one), and per run its destination.
+// Per iteration
+//   gather: a CTA takes a task (a range of chunks of one block), loads the
+//     block's contributions into shared memory, streams the chunks, sums each
+//     run (8 arcs per lane, runs that span lanes by a segmented warp sum) and
+//     adds the runs' sums to their destinations with reductions that return
+//     nothing (32 consecutive runs at a time: ascending destinations);
 //   finish: per vertex the new rank and its contribution (coalesced).
-// Against the row sweep, an arc costs 3 streamed bytes instead of a 4-byte
-// column and a 4-byte random gather, and one contribution is gathered per
-// run instead of per arc (0.16 runs per arc on RMAT graphs in degree order
-// at 4 M vertices).  Measured on RMAT-24: 18.9 ms for 15 iterations against
-// 29.3 ms for pr_pull_flat.  Variants that wrote each contribution into the
-// slots of its runs (so the gather read them sequentially) were slower
-// (23-35 ms): the scattered 4-byte writes into a 0.5 GB array cost more than
-// the gathers from the L2-resident contributions.
+// An arc costs 2.1 streamed bytes and one shared-memory read, a run 4 bytes
+// and one reduction in L2 (0.16 runs per arc on RMAT graphs in degree order at
+// 4 M vertices).  The reverse, destinations cut into blocks with their sums in
+// shared memory and one contribution gathered per run, adds every arc with a
+// shared-memory atomic: RMAT-23 symmetric (15 iterations) 10.6 ms, 10.0 with
+// each chunk's contributions staged in shared memory, against 8.1 here (0.54 ms
+// an iteration, 470 G arcs/s; RMAT-21 of edge factor 8 3.2 -> 1.8), and the
+// sort by block of sources alone builds the layout in 18 ms instead of 65.
+// Bound by instruction issue and the shared-memory reads of the gather (about
+// four fifths) and by the vertex pass.
 
-constexpr uint32_t kBinPart = 32768;  // destinations per partition (a local id fits 15 bits)
-constexpr uint32_t kBinChunk = 256;   // arcs per chunk (a run offset fits a byte)
+constexpr uint32_t kBinPart = 32768;  // sources per block (a local id fits 16 bits, with kBinPart for padding)
+constexpr uint32_t kBinChunk = 256;   // arcs per chunk
 constexpr int kBinBlock = 1024;
-constexpr uint16_t kBinPad = 0xFFFFu;
+// A row gets one addition per block of sources and chunk.  In 32 bits the
+// largest ranks' rounding put the result 3.6e-7 of its norm off at RMAT-23
+// (2.7e-7 with the sums built in shared memory), so the kBinHubs largest rows
+// are added up in 64 bits: 6e-8; 4096 rows 1.4e-7.  All heavy rows: 4e-8, but
+// the conversions of every run's sum cost 0.2 ms an iteration.
+constexpr uint32_t kBinHubs = 16384;
+// Shared memory of the gather: the block's contributions, a zero for padding,
+// then per warp a chunk's run sums.
+constexpr size_t kBinSmem = sizeof(float) * (kBinPart + 32 + kBinBlock / 32 * kBinChunk);
 
-// A lane's 8 arcs of chunk c (all padding past the task's end).
-__device__ __forceinline__ void bin_load_chunk(const PrArgs& a, uint64_t c, uint64_t cend, uint32_t lane, uint4& dd,
-                                               uint2& rr, uint32_t& r0) {
+// A lane's 8 arcs of chunk c and their run flags (nothing past the task's end).
+__device__ __forceinline__ void bin_load_chunk(const PrArgs& a, uint64_t c, uint64_t cend, uint32_t lane, uint4& u,
+                                               uint32_t& f) {
+  u = make_uint4(0u, 0u, 0u, 0u);
+  f = 0u;
   if (c < cend) {
-    dd = ldg(reinterpret_cast<const uint4*>(a.b_dst + c * kBinChunk) + lane);
-    rr = ldg(reinterpret_cast<const uint2*>(a.b_roff + c * kBinChunk) + lane);
-    r0 = ldg(a.b_crun + c);
-  } else {
-    dd = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-    rr = make_uint2(0u, 0u);
-    r0 = 0u;
+    u = ldg(reinterpret_cast<const uint4*>(a.b_src + c * kBinChunk) + lane);
+    f = ldg(a.b_flag + c * (kBinChunk / 8) + lane);
   }
 }
 
-__device__ __forceinline__ uint32_t bin_dst(const uint4& dd, int k) {
-  const uint32_t w = k < 2 ? dd.x : k < 4 ? dd.y : k < 6 ? dd.z : dd.w;
-  return (w >> (16 * (k & 1))) & 0xFFFFu;
+// The runs of chunk c: the first and their number.
+__device__ __forceinline__ uint2 bin_runs(const PrArgs& a, uint64_t c, uint64_t cend) {
+  if (c >= cend) return make_uint2(0u, 0u);
+  const uint32_t r = ldg(a.b_crun + c);
+  return make_uint2(r, ldg(a.b_crun + c + 1) - r);
 }
 
-// The contributions of a lane's 8 arcs: each run's source, then its
-// contribution (written by the finish pass: a plain load, not ldg; the
-// 64 MB of contributions at 16 M vertices stay mostly in L2).
-__device__ __forceinline__ void bin_load_vals(const PrArgs& a, const float* c_in, const uint4& dd, const uint2& rr,
-                                              uint32_t r0, float (&x)[8]) {
-  uint32_t u[8];
+// The destinations of a chunk's first 64 runs, two per lane.
+__device__ __forceinline__ uint2 bin_dests(const PrArgs& a, uint2 runs, uint32_t lane) {
+  return make_uint2(lane < runs.y ? ldg(a.b_rdst + runs.x + lane) : 0u,
+                    lane + 32 < runs.y ? ldg(a.b_rdst + runs.x + lane + 32) : 0u);
+}
+
+// The sums of a chunk's runs into s_run.  All lanes call.
+__device__ __forceinline__ void bin_run_sums(const float* s_c, uint4 u, uint32_t f, uint32_t lane, float* s_run) {
+  uint32_t upto = __popc(f);  // runs that start in this lane or before it
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, upto, o);
+    if (lane >= (uint32_t)o) upto += y;
+  }
+  float x[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const uint32_t off = ((k < 4 ? rr.x : rr.y) >> (8 * (k & 3))) & 0xFFu;
-    u[k] = bin_dst(dd, k) != kBinPad ? ldg(a.b_rsrc + r0 + off) : 0xFFFFFFFFu;
+    const uint32_t w = k < 2 ? u.x : k < 4 ? u.y : k < 6 ? u.z : u.w;
+    x[k] = s_c[(w >> (16 * (k & 1))) & 0xFFFFu];
   }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) x[k] = u[k] != 0xFFFFFFFFu ? c_in[u[k]] : 0.f;
-}
-
-// Add a lane's 8 arcs into the partition sums, one atomic per distinct
-// destination (the 8 are sorted by destination, padding last).  A lane's
-// last destination may continue in the next lanes (the chunk is sorted), so
-// those last runs are first summed over the warp by destination: a chunk of
-// 256 arcs into one hub makes one atomic, not 32, and the hub's sum is built
-// from tree-summed parts (32 sequential float adds per chunk lost 8e-5 of a
-// hub's rank over 150 K in-arcs).  All lanes call.
-__device__ __forceinline__ void bin_add(float* s_sum, const uint4& dd, const float (&x)[8]) {
-  uint32_t cur = bin_dst(dd, 0);
-  float run = x[0];
+  // runs that start and end here are stored; the arcs before the lane's first
+  // start belong to a run of the lanes before, the ones from its last start on
+  // to one that may go on in the next lanes
+  uint32_t r = upto - __popc(f);  // the next run to start here
+  float sum = x[0], head = 0.f;
+  bool started = f & 1u;
+  r += started;
 #pragma unroll
   for (int k = 1; k < 8; ++k) {
-    const uint32_t d = bin_dst(dd, k);
-    if (d != cur) {
-      if (cur != kBinPad && run != 0.f) atomicAdd(&s_sum[cur], run);
-      cur = d;
-      run = x[k];
+    if ((f >> k) & 1u) {
+      if (started) s_run[r - 1] = sum;
+      else head = sum;
+      started = true;
+      ++r;
+      sum = x[k];
     } else {
-      run += x[k];
+      sum += x[k];
     }
   }
-  // only when some lane's last destination continues in the next lane
-  const uint32_t next_first = __shfl_down_sync(kFull, bin_dst(dd, 0), 1);
-  const bool cont = (threadIdx.x & 31u) < 31u && cur != kBinPad && next_first == cur;
-  if (__any_sync(kFull, cont)) {
-    if (seg_reduce(cur != kBinPad, cur, run) && run != 0.f) atomicAdd(&s_sum[cur], run);
-  } else if (cur != kBinPad && run != 0.f) {
-    atomicAdd(&s_sum[cur], run);
-  }
+  const float next = __shfl_down_sync(kFull, head, 1);
+  if (lane < 31) sum += next;
+  // a lane without a start only continues the run of the lanes before it
+  if (__any_sync(kFull, f == 0)) seg_reduce(true, upto, sum);
+  if (f) s_run[upto - 1] = sum;
 }
 
 // The gather phase of a binned iteration: the CTA takes tasks until none is
-// left and leaves in every destination's sum slot of acc_cur the sum of
-// c_in over its in-arcs.  All threads of the CTA call.
+// left and adds to acc_cur (zero before) the sums of c_in over the in-arcs.
+// All threads of the CTA call.
 template <int BLOCK>
-__device__ __forceinline__ void bin_gather(const PrArgs& a, const float* c_in, float* acc_cur, uint32_t it, float* s_sum,
-                                           uint32_t* s_task) {
+__device__ __forceinline__ void bin_gather(const PrArgs& a, const float* c_in, float* acc_cur, double* hacc_cur,
+                                           uint32_t it, float* s_c, uint32_t* s_task) {
   const uint32_t tid = threadIdx.x, lane = lane_id(), wib = tid >> 5;
   constexpr uint32_t kW = BLOCK / 32;
-    for (;;) {
-      if (tid == 0) *s_task = atomicAdd(&a.ctl->task_next[it & 1], 1u);
-      __syncthreads();
-      const uint32_t t = *s_task;
-      if (t >= a.b_ntasks) break;  // uniform
-      const uint4 tk = ldg(a.b_tasks + t);
-      const uint32_t v0 = tk.x, nv = tk.y & 0x7FFFFFFFu;
-      const bool multi = (tk.y >> 31) != 0u;
-      for (uint32_t d = tid; d < nv; d += BLOCK) s_sum[d] = 0.f;
-      __syncthreads();
-      // a lane takes 8 consecutive arcs of a chunk (sorted by destination
-      // inside the chunk, so equal destinations are summed in registers
-      // before one shared-memory atomic); the next chunk's words load while
-      // this chunk's contributions are read and added (a second chunk ahead
-      // measured slower: 29.6 against 23.0 ms on RMAT-24)
-      uint64_t c = tk.z + wib;
-      uint4 dd;
-      uint2 rr;
-      uint32_t r0;
-      bin_load_chunk(a, c, tk.w, lane, dd, rr, r0);
-      for (; c < tk.w; c += kW) {
-        uint4 ddn;
-        uint2 rrn;
-        uint32_t r0n;
-        bin_load_chunk(a, c + kW, tk.w, lane, ddn, rrn, r0n);
-        float x[8];
-        bin_load_vals(a, c_in, dd, rr, r0, x);
-        bin_add(s_sum, dd, x);
-        dd = ddn;
-        rr = rrn;
-        r0 = r0n;
+  static_assert(BLOCK == 1024, "a lane per warp adds up the warps' chunks of one run");
+  __shared__ uint32_t s_hub[kW];
+  __shared__ double s_hsum[kW];
+  auto add = [&](uint32_t v, float x) {
+    if (x == 0.f) return;
+    if (v < a.b_nheavy) atomicAdd(&hacc_cur[v], (double)x);
+    else atomicAdd(&acc_cur[v], x);
+  };
+  auto add_hub = [&](uint32_t v, double x) {
+    if (x == 0.0) return;
+    if (v < a.b_nheavy) atomicAdd(&hacc_cur[v], x);
+    else atomicAdd(&acc_cur[v], (float)x);
+  };
+  float* s_run = s_c + kBinPart + 32 + wib * kBinChunk;
+  if (tid == 0) s_c[kBinPart] = 0.f;
+  for (;;) {
+    if (tid == 0) *s_task = atomicAdd(&a.ctl->task_next[it & 1], 1u);
+    __syncthreads();
+    const uint32_t t = *s_task;
+    if (t >= a.b_ntasks) break;  // uniform
+    const uint4 tk = ldg(a.b_tasks + t);
+    // written by the finish pass: plain loads, not ldg
+    const float4* c4 = reinterpret_cast<const float4*>(c_in + tk.x);  // a multiple of kBinPart
+#pragma unroll 4
+    for (uint32_t d = tid; d < tk.y / 4; d += BLOCK) reinterpret_cast<float4*>(s_c)[d] = c4[d];
+    for (uint32_t d = (tk.y & ~3u) + tid; d < tk.y; d += BLOCK) s_c[d] = c_in[tk.x + d];
+    __syncthreads();
+    // loaded ahead: a chunk's runs two chunks before it is summed, its arcs and
+    // the runs' destinations one
+    uint64_t c = tk.z + wib;
+    const uint64_t cend = tk.w;
+    uint4 u;
+    uint32_t f;
+    bin_load_chunk(a, c, cend, lane, u, f);
+    uint2 r0 = bin_runs(a, c, cend), r1 = bin_runs(a, c + kW, cend);
+    uint2 d0 = bin_dests(a, r0, lane);
+    // whole chunks of one destination are summed over the task before they are
+    // added: a hub's sum takes one addition per task, not one per chunk
+    uint32_t hub = 0xFFFFFFFFu;
+    double hsum = 0.0;
+    for (; c < cend; c += kW) {
+      uint4 un;
+      uint32_t fn;
+      bin_load_chunk(a, c + kW, cend, lane, un, fn);
+      const uint2 d1 = bin_dests(a, r1, lane), r2 = bin_runs(a, c + 2 * kW, cend);
+      bin_run_sums(s_c, u, f, lane, s_run);
+      __syncwarp();
+      if (r0.y == 1) {
+        const uint32_t v = __shfl_sync(kFull, d0.x, 0);
+        if (v != hub) {
+          if (lane == 0) add_hub(hub, hsum);  // nothing the first time
+          hub = v;
+          hsum = 0.0;
+        }
+        hsum += s_run[0];
+        r0.y = 0;
       }
-      __syncthreads();
-      for (uint32_t d = tid; d < nv; d += BLOCK) {
-        const float x = s_sum[d];
-        if (!multi) acc_cur[v0 + d] = x;
-        else if (x != 0.f) atomicAdd(&acc_cur[v0 + d], x);
+      if (lane < r0.y) add(d0.x, s_run[lane]);
+      if (lane + 32 < r0.y) add(d0.y, s_run[lane + 32]);
+#pragma unroll 2
+      for (uint32_t k = 64 + lane; k < r0.y; k += 32) {
+        add(ldg(a.b_rdst + r0.x + k), s_run[k]);
       }
-      __syncthreads();  // s_sum and s_task are reused by the next task
+      __syncwarp();  // s_run is rewritten by the next chunk
+      u = un, f = fn;
+      r0 = r1, r1 = r2, d0 = d1;
     }
+    if (lane == 0) {
+      s_hub[wib] = hub;
+      s_hsum[wib] = hsum;
+    }
+    __syncthreads();  // s_c and s_task are reused by the next task
+    if (wib == 0) {
+      const uint32_t v = s_hub[lane];
+      const double x = s_hsum[lane];
+      for (unsigned left = __ballot_sync(kFull, v != 0xFFFFFFFFu); left;) {
+        const uint32_t w = __shfl_sync(kFull, v, __ffs(left) - 1);
+        const double sum = warp_sum(v == w ? x : 0.0);
+        if (lane == 0) add_hub(w, sum);
+        left &= ~__ballot_sync(kFull, v == w);
+      }
+    }
+  }
 }
 
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) pr_pull_binned(PrArgs a) {
-  extern __shared__ float s_sum[];  // kBinPart floats
+  extern __shared__ __align__(16) float s_c[];  // kBinSmem bytes
   __shared__ double s_l1, s_total;
   __shared__ uint32_t s_max, s_task;
   if (threadIdx.x == 0) {
@@ -641,34 +694,54 @@ __global__ void __launch_bounds__(BLOCK, 1) pr_pull_binned(PrArgs a) {
   __syncthreads();
   PrCtl* ctl = a.ctl;
   const uint64_t deadline = kernel_deadline();
-  const uint32_t tid = threadIdx.x, lane = lane_id(), wib = tid >> 5;
-  constexpr uint32_t kW = BLOCK / 32;
-  const uint64_t gtid = blockIdx.x * (uint64_t)BLOCK + tid;
+  const uint64_t gtid = blockIdx.x * (uint64_t)BLOCK + threadIdx.x;
   const uint64_t gthreads = (uint64_t)gridDim.x * BLOCK;
   float* const c_io = a.c[0];  // gathered, then rewritten after the barrier
   for (uint32_t it = 0;; ++it) {
     float* const acc_cur = (it & 1) ? a.acc2 : a.acc;
     float* const acc_nxt = (it & 1) ? a.acc : a.acc2;
+    double* const hacc_cur = a.hacc + (it & 1) * a.b_nheavy;
+    double* const hacc_nxt = a.hacc + ((it + 1) & 1) * a.b_nheavy;
     if (gtid == 0) {
       clear_change(ctl, (it + 1) % 3);
       ctl->task_next[(it + 1) & 1] = 0u;  // the counter iteration it + 1 takes (it - 1's is done)
     }
-    bin_gather<BLOCK>(a, c_io, acc_cur, it, s_sum, &s_task);
+    bin_gather<BLOCK>(a, c_io, acc_cur, hacc_cur, it, s_c, &s_task);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     // ---- finish: ranks and contributions for the next gather
     double my_l1 = 0.0;
     float my_max = 0.f;
     const uint32_t vend = it >= 2 ? a.zero_from : a.n;  // constant tail skipped (its values stay)
-    for (uint64_t v = gtid; v < vend; v += gthreads) {
-      const float sum = acc_cur[v];
-      acc_nxt[v] = 0.f;
+    auto finish = [&](uint64_t v, float sum, float old, uint32_t k) {
       const float value = sum * a.alpha + a.base;  // PageRank-pull.cpp:222
-      const float old = a.value[v];
       a.value[v] = value;
-      const uint32_t k = a.nout[v];
       c_io[v] = k ? value / (float)k : 0.f;
       my_l1 += (double)fabsf(value - old);
       my_max = fmaxf(my_max, fabsf(value - old));
+    };
+    const uint32_t nh = min(a.b_nheavy, vend);
+    for (uint64_t v = gtid; v < nh; v += gthreads) {
+      const double sum = hacc_cur[v];
+      hacc_nxt[v] = 0.0;
+      finish(v, (float)sum, a.value[v], a.nout[v]);
+    }
+    // four vertices' loads together, as no load may pass the stores (one
+    // vertex at a time: 0.77 ms an iteration of RMAT-23, not 0.54)
+    for (uint64_t v0 = nh + gtid; v0 < vend; v0 += 4 * gthreads) {
+      float sum[4], old[4];
+      uint32_t k[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t v = v0 + j * gthreads;
+        if (v < vend) sum[j] = acc_cur[v], old[j] = a.value[v], k[j] = a.nout[v];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t v = v0 + j * gthreads;
+        if (v >= vend) break;
+        acc_nxt[v] = 0.f;
+        finish(v, sum[j], old[j], k[j]);
+      }
     }
     publish_change(ctl, it % 3, my_l1, my_max, &s_l1, &s_max);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
@@ -678,67 +751,93 @@ __global__ void __launch_bounds__(BLOCK, 1) pr_pull_binned(PrArgs a) {
   }
 }
 
-// Layout build, once per graph.  key = partition << 32 | source, value = destination.
+// Layout build, once per graph: arcs per block of sources, then per arc its
+// block (the sort key) and destination << 16 | local source.
+__global__ void bin_count_kernel(const uint32_t* __restrict__ nout, uint32_t n, unsigned long long* __restrict__ count) {
+  const uint64_t v0 = (uint64_t)blockIdx.x * kBinPart, v1 = min(v0 + kBinPart, (uint64_t)n);
+  unsigned long long mine = 0;
+  for (uint64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) mine += nout[v];
+  mine = warp_sum(mine);
+  if (lane_id() == 0 && mine) atomicAdd(&count[blockIdx.x], mine);
+}
+
 __global__ void bin_keys_kernel(const uint64_t* __restrict__ offs, const uint32_t* __restrict__ col, uint32_t n,
-                                uint64_t* __restrict__ key, uint32_t* __restrict__ row) {
+                                uint16_t* __restrict__ key, uint64_t* __restrict__ val) {
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint32_t lane = lane_id();
   for (uint64_t v = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
-    const uint64_t p = v / kBinPart;
     for (uint64_t j = offs[v] + lane; j < offs[v + 1]; j += 32) {
-      key[j] = (p << 32) | col[j];
-      row[j] = (uint32_t)v;
+      const uint32_t u = col[j];
+      key[j] = (uint16_t)(u / kBinPart);
+      val[j] = v << 16 | u % kBinPart;
     }
   }
 }
 
-// runs: 1 where a (partition, source) pair starts
-__global__ void bin_flags_kernel(const uint64_t* __restrict__ key, uint64_t m, uint32_t* __restrict__ flag) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride)
-    flag[i] = (i == 0 || key[i] != key[i - 1]) ? 1u : 0u;
+// A warp's chunk of the sorted arcs (arcs first[p] .. of block p fill the
+// chunks from pad[p] / kBinChunk on): its lane's 8 destinations and local
+// sources (kBinPart past the block's end) and the byte of run starts.
+__device__ __forceinline__ uint32_t bin_chunk_arcs(const uint64_t* __restrict__ val, const uint64_t* __restrict__ first,
+                                                   const uint64_t* __restrict__ pad, uint32_t P, uint64_t c,
+                                                   uint32_t (&dst)[8], uint32_t (&src)[8]) {
+  uint32_t lo = 0, hi = P;  // the last block that starts at or before the chunk and is not empty
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) / 2;
+    if (pad[mid] <= c * kBinChunk) lo = mid;
+    else hi = mid;
+  }
+  const uint32_t lane = lane_id();
+  const uint64_t i = first[lo] + (c * kBinChunk - pad[lo]) + lane * 8;
+  const uint64_t e = first[lo + 1];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const bool ok = i + k < e;
+    const uint64_t x = ok ? val[i + k] : 0ull;
+    dst[k] = (uint32_t)(x >> 16);
+    src[k] = ok ? (uint32_t)x & 0xFFFFu : kBinPart;
+  }
+  const uint32_t before = __shfl_up_sync(kFull, dst[7], 1);
+  uint32_t f = (lane == 0 || (i < e && dst[0] != before)) ? 1u : 0u;
+#pragma unroll
+  for (int k = 1; k < 8; ++k)
+    if (i + k < e && dst[k] != dst[k - 1]) f |= 1u << k;
+  return f;
 }
 
-// Sorted arc i of partition p goes to padded position pad[p] + i - first[p].
-__global__ void bin_place_kernel(const uint64_t* __restrict__ key, const uint32_t* __restrict__ row,
-                                 const uint32_t* __restrict__ runp1, uint64_t m, const uint64_t* __restrict__ first,
-                                 const uint64_t* __restrict__ pad, uint16_t* __restrict__ dst,
-                                 uint32_t* __restrict__ crun, uint32_t* __restrict__ run_src) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
-    const uint32_t p = (uint32_t)(key[i] >> 32);
-    const uint64_t q = pad[p] + (i - first[p]);
-    dst[q] = (uint16_t)(row[i] % kBinPart);
-    const uint32_t r = runp1[i] - 1;
-    if (q % kBinChunk == 0) crun[q / kBinChunk] = r;
-    if (i == 0 || runp1[i] != runp1[i - 1]) run_src[r] = (uint32_t)key[i];
+__global__ void bin_place_kernel(const uint64_t* __restrict__ val, const uint64_t* __restrict__ first,
+                                 const uint64_t* __restrict__ pad, uint32_t P, uint64_t nchunks, uint16_t* __restrict__ src,
+                                 uint8_t* __restrict__ flag, uint32_t* __restrict__ count) {
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint32_t lane = lane_id();
+  for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nw) {
+    uint32_t d[8], u[8];
+    const uint32_t f = bin_chunk_arcs(val, first, pad, P, c, d, u);
+    reinterpret_cast<uint4*>(src + c * kBinChunk)[lane] =
+        make_uint4(u[0] | u[1] << 16, u[2] | u[3] << 16, u[4] | u[5] << 16, u[6] | u[7] << 16);
+    flag[c * (kBinChunk / 8) + lane] = (uint8_t)f;
+    const uint32_t runs = __reduce_add_sync(kFull, __popc(f));
+    if (lane == 0) count[c] = runs;
   }
 }
 
-__global__ void bin_roff_kernel(const uint64_t* __restrict__ key, const uint32_t* __restrict__ runp1, uint64_t m,
-                                const uint64_t* __restrict__ first, const uint64_t* __restrict__ pad,
-                                const uint32_t* __restrict__ crun, uint8_t* __restrict__ roff) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += stride) {
-    const uint32_t p = (uint32_t)(key[i] >> 32);
-    const uint64_t q = pad[p] + (i - first[p]);
-    roff[q] = (uint8_t)(runp1[i] - 1 - crun[q / kBinChunk]);
-  }
-}
-
-// Sort each chunk's arcs by destination (padding last): equal destinations
-// become neighbours, so a lane sums them before its atomic.
-__global__ void __launch_bounds__(kBinChunk) bin_chunk_sort_kernel(uint16_t* __restrict__ dst, uint8_t* __restrict__ roff,
-                                                                   uint64_t nchunks) {
-  using Sort = cub::BlockRadixSort<uint32_t, kBinChunk, 1>;
-  __shared__ typename Sort::TempStorage tmp;
-  for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    const uint64_t i = c * kBinChunk + threadIdx.x;
-    uint32_t key[1] = {((uint32_t)dst[i] << 8) | roff[i]};
-    Sort(tmp).Sort(key, 0, 24);
-    dst[i] = (uint16_t)(key[0] >> 8);
-    roff[i] = (uint8_t)(key[0] & 0xFFu);
-    __syncthreads();  // the temp storage is reused by the next chunk
+__global__ void bin_runs_kernel(const uint64_t* __restrict__ val, const uint64_t* __restrict__ first,
+                                const uint64_t* __restrict__ pad, uint32_t P, uint64_t nchunks,
+                                const uint32_t* __restrict__ crun, uint32_t* __restrict__ rdst) {
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint32_t lane = lane_id();
+  for (uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nw) {
+    uint32_t d[8], u[8];
+    const uint32_t f = bin_chunk_arcs(val, first, pad, P, c, d, u);
+    uint32_t upto = __popc(f);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, upto, o);
+      if (lane >= (uint32_t)o) upto += y;
+    }
+    uint32_t r = crun[c] + upto - __popc(f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if ((f >> k) & 1u) rdst[r++] = d[k];
   }
 }
 
@@ -781,14 +880,18 @@ __device__ __forceinline__ void resid_vertex_pass(const PrArgs& a, uint32_t it, 
   uint32_t my_accum = 0;
   for (uint64_t v = gtid; v < a.n; v += gthreads) {
     float r = a.residual[v];
-    if (it > 0) {
-      const float sum = acc_prev[v];
-      if (sum > 0.f) r = sum;
-    }
     // the sums of round it - 2, read by round it - 1: zeroed for this
     // round's gather (zeroing the slots the last gather's atomics just
     // updated stalls)
-    acc_cur[v] = 0.f;
+    float sum;
+    if (v < a.b_nheavy) {
+      sum = (float)a.hacc[((it + 1) & 1) * a.b_nheavy + v];
+      a.hacc[(it & 1) * a.b_nheavy + v] = 0.0;
+    } else {
+      sum = acc_prev[v];
+      acc_cur[v] = 0.f;
+    }
+    if (it > 0 && sum > 0.f) r = sum;
     float d = 0.f;
     if (r > a.tol) {
       a.value[v] += r;
@@ -858,7 +961,7 @@ __global__ void __launch_bounds__(kBlock, 6) pr_pull_residual_persistent(PrArgs 
 // The same rounds over the binned layout (degree-ordered graphs).
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1) pr_resid_binned(PrArgs a) {
-  extern __shared__ float s_sum[];  // kBinPart floats
+  extern __shared__ __align__(16) float s_c[];  // kBinSmem bytes
   __shared__ uint32_t s_task;
   PrCtl* ctl = a.ctl;
   const uint64_t deadline = kernel_deadline();
@@ -873,7 +976,7 @@ __global__ void __launch_bounds__(BLOCK, 1) pr_resid_binned(PrArgs a) {
     }
     resid_vertex_pass(a, it, acc_prev, acc_cur, gtid, gthreads);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-    bin_gather<BLOCK>(a, a.delta, acc_cur, it, s_sum, &s_task);
+    bin_gather<BLOCK>(a, a.delta, acc_cur, a.hacc + (it & 1) * a.b_nheavy, it, s_c, &s_task);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
     const uint32_t accum = *reinterpret_cast<volatile uint32_t*>(&ctl->active[it % 3]);
     if (gtid == 0) ctl->iters = it + 1;
@@ -1219,55 +1322,22 @@ int ensure_pr_bins(gb_graph* g, cudaStream_t s) {
   if (g->prb) return GB_OK;
   const uint32_t n = g->n;
   const uint64_t m = g->m;
-  if (m == 0 || m >= 0xFFFFFFF0ull) return GB_ERR_UNSUPPORTED;  // run ids and run offsets are 32-bit
   const uint32_t P = (uint32_t)(((uint64_t)n + kBinPart - 1) / kBinPart);
-  std::vector<uint64_t> ho((size_t)n + 1);
-  GB_CUDA(cudaMemcpyAsync(ho.data(), g->offs, sizeof(uint64_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost, s));
-  GB_CUDA(cudaStreamSynchronize(s));
-  // partitions: their arcs, padded to whole chunks; tasks of about
-  // m / (6 per SM) arcs, the largest first
-  std::vector<uint64_t> first((size_t)P + 1), pad((size_t)P + 1);
-  uint64_t mpad = 0;
-  for (uint32_t p = 0; p < P; ++p) {
-    const uint64_t v0 = (uint64_t)p * kBinPart, v1 = std::min<uint64_t>(v0 + kBinPart, n);
-    first[p] = ho[v0];
-    pad[p] = mpad;
-    mpad += (ho[v1] - ho[v0] + kBinChunk - 1) / kBinChunk * kBinChunk;
-  }
-  first[P] = m;
-  pad[P] = mpad;
-  const uint64_t nchunks = mpad / kBinChunk;
-  const uint64_t target_chunks = std::max<uint64_t>(64, m / ((uint64_t)g->sm_count * 6 * kBinChunk));
-  std::vector<uint4> tasks;
-  for (uint32_t p = 0; p < P; ++p) {
-    const uint64_t c0 = pad[p] / kBinChunk, c1 = pad[p + 1] / kBinChunk;
-    if (c0 == c1) continue;  // no in-arcs: the finish pass keeps those sums at zero
-    const uint64_t nt = (c1 - c0 + target_chunks - 1) / target_chunks;
-    const uint64_t per = (c1 - c0 + nt - 1) / nt;
-    const uint32_t v0 = p * kBinPart;
-    const uint32_t nv = (uint32_t)std::min<uint64_t>(kBinPart, (uint64_t)n - v0);
-    for (uint64_t c = c0; c < c1; c += per)
-      tasks.push_back(make_uint4(v0, nv | (nt > 1 ? 0x80000000u : 0u), (uint32_t)c, (uint32_t)std::min(c1, c + per)));
-  }
-  std::stable_sort(tasks.begin(), tasks.end(), [](const uint4& x, const uint4& y) { return x.w - x.z > y.w - y.z; });
-  if (nchunks >= 0xFFFFFFFFull) return GB_ERR_UNSUPPORTED;  // chunk ids are 32-bit in the tasks
-
-  // temporaries
-  uint64_t *key0 = nullptr, *key1 = nullptr, *dfirst = nullptr;
-  uint32_t *row0 = nullptr, *row1 = nullptr, *runp1 = nullptr;
+  if (m == 0 || m >= 0xFFFFFFF0ull || P > 65536) return GB_ERR_UNSUPPORTED;  // run ids are 32-bit, block ids 16-bit
+  uint16_t *key0 = nullptr, *key1 = nullptr;
+  uint64_t *val0 = nullptr, *val1 = nullptr, *dfirst = nullptr;
   void* tmp = nullptr;
-  size_t tmp_bytes = 0;
   PrBins* b = new PrBins;
   auto cleanup = [&](bool keep) {
     cudaFree(key0);
     cudaFree(key1);
-    cudaFree(row0);
-    cudaFree(row1);
-    cudaFree(runp1);
+    cudaFree(val0);
+    cudaFree(val1);
     cudaFree(dfirst);
     cudaFree(tmp);
     if (!keep) {
       cudaFree(b->mem);
+      cudaFree(b->rdst);
       delete b;
     }
   };
@@ -1280,61 +1350,89 @@ int ensure_pr_bins(gb_graph* g, cudaStream_t s) {
       return _st;                           \
     }                                       \
   } while (0)
-  GB_BTRY(cudaMalloc(&key0, sizeof(uint64_t) * m));
-  GB_BTRY(cudaMalloc(&key1, sizeof(uint64_t) * m));
-  GB_BTRY(cudaMalloc(&row0, sizeof(uint32_t) * m));
-  GB_BTRY(cudaMalloc(&row1, sizeof(uint32_t) * m));
-  GB_BTRY(cudaMalloc(&runp1, sizeof(uint32_t) * m));
   GB_BTRY(cudaMalloc(&dfirst, sizeof(uint64_t) * 2 * ((size_t)P + 1)));
   uint64_t* dpad = dfirst + P + 1;
+  std::vector<uint64_t> first((size_t)P + 1), pad((size_t)P + 1);
+  GB_BTRY(cudaMemsetAsync(dpad, 0, sizeof(uint64_t) * P, s));
+  bin_count_kernel<<<P, 256, 0, s>>>(g->outdeg_of_stored, n, reinterpret_cast<unsigned long long*>(dpad));
+  GB_BTRY(cudaGetLastError());
+  GB_BTRY(cudaMemcpyAsync(pad.data(), dpad, sizeof(uint64_t) * P, cudaMemcpyDeviceToHost, s));
+  GB_BTRY(cudaStreamSynchronize(s));
+  // blocks: their arcs, padded to whole chunks; tasks of about
+  // m / (6 per SM) arcs, the largest first
+  uint64_t at = 0, mpad = 0;
+  for (uint32_t p = 0; p < P; ++p) {
+    const uint64_t cnt = pad[p];
+    first[p] = at;
+    pad[p] = mpad;
+    at += cnt;
+    mpad += (cnt + kBinChunk - 1) / kBinChunk * kBinChunk;
+  }
+  first[P] = at;
+  pad[P] = mpad;
+  const uint64_t nchunks = mpad / kBinChunk;
+  if (at != m || nchunks >= 0xFFFFFFFEull) {  // chunk ids are 32-bit in the tasks
+    cleanup(false);
+    return GB_ERR_UNSUPPORTED;
+  }
+  const uint64_t target_chunks = std::max<uint64_t>(64, m / ((uint64_t)g->sm_count * 6 * kBinChunk));
+  std::vector<uint4> tasks;
+  for (uint32_t p = 0; p < P; ++p) {
+    const uint64_t c0 = pad[p] / kBinChunk, c1 = pad[p + 1] / kBinChunk;
+    if (c0 == c1) continue;  // sources without out-arcs
+    const uint64_t nt = (c1 - c0 + target_chunks - 1) / target_chunks;
+    const uint64_t per = (c1 - c0 + nt - 1) / nt;
+    const uint32_t v0 = p * kBinPart;
+    const uint32_t nv = (uint32_t)std::min<uint64_t>(kBinPart, (uint64_t)n - v0);
+    for (uint64_t c = c0; c < c1; c += per)
+      tasks.push_back(make_uint4(v0, nv, (uint32_t)c, (uint32_t)std::min(c1, c + per)));
+  }
+  std::stable_sort(tasks.begin(), tasks.end(), [](const uint4& x, const uint4& y) { return x.w - x.z > y.w - y.z; });
+
+  GB_BTRY(cudaMalloc(&key0, sizeof(uint16_t) * m));
+  GB_BTRY(cudaMalloc(&key1, sizeof(uint16_t) * m));
+  GB_BTRY(cudaMalloc(&val0, sizeof(uint64_t) * m));
+  GB_BTRY(cudaMalloc(&val1, sizeof(uint64_t) * m));
   GB_BTRY(cudaMemcpyAsync(dfirst, first.data(), sizeof(uint64_t) * ((size_t)P + 1), cudaMemcpyHostToDevice, s));
   GB_BTRY(cudaMemcpyAsync(dpad, pad.data(), sizeof(uint64_t) * ((size_t)P + 1), cudaMemcpyHostToDevice, s));
   const int grid = g->sm_count * 8;
-  bin_keys_kernel<<<grid, 256, 0, s>>>(g->offs, g->col, n, key0, row0);
+  bin_keys_kernel<<<grid, 256, 0, s>>>(g->offs, g->col, n, key0, val0);
   GB_BTRY(cudaGetLastError());
-  int end_bit = 33;  // partition ids above the 32 source bits
-  while ((1ull << (end_bit - 32)) < (uint64_t)P) ++end_bit;
-  cub::DoubleBuffer<uint64_t> dk(key0, key1);
-  cub::DoubleBuffer<uint32_t> dv(row0, row1);
+  // stable: the rows' order (by destination) stays inside a block
+  int end_bit = 1;
+  while ((1u << end_bit) < P) ++end_bit;
+  cub::DoubleBuffer<uint16_t> dk(key0, key1);
+  cub::DoubleBuffer<uint64_t> dv(val0, val1);
+  // the cached layout but the runs' destinations, one allocation (parts 256-byte aligned)
+  auto part = [](uint64_t bytes) { return (bytes + 255) & ~uint64_t(255); };
+  const uint64_t sz_src = part(2 * mpad), sz_flag = part(mpad / 8), sz_crun = part(4 * (nchunks + 1)),
+                 sz_tasks = part(16 * tasks.size());
+  GB_BTRY(cudaMalloc(&b->mem, sz_src + sz_flag + sz_crun + sz_tasks));
+  char* q = static_cast<char*>(b->mem);
+  b->src = reinterpret_cast<uint16_t*>(q);
+  q += sz_src;
+  b->flag = reinterpret_cast<uint8_t*>(q);
+  q += sz_flag;
+  b->crun = reinterpret_cast<uint32_t*>(q);
+  q += sz_crun;
+  b->tasks = reinterpret_cast<uint4*>(q);
+  b->ntasks = (uint32_t)tasks.size();
+  size_t tmp_bytes = 0, scan_bytes = 0;
   GB_BTRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, dk, dv, (int64_t)m, 0, end_bit, s));
-  size_t scan_bytes = 0;
-  GB_BTRY(cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, runp1, runp1, (int64_t)m, s));
+  GB_BTRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, b->crun, b->crun, (int64_t)(nchunks + 1), s));
   tmp_bytes = std::max(tmp_bytes, scan_bytes);
   GB_BTRY(cudaMalloc(&tmp, std::max<size_t>(tmp_bytes, 16)));
   GB_BTRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, dk, dv, (int64_t)m, 0, end_bit, s));
-  bin_flags_kernel<<<grid, 256, 0, s>>>(dk.Current(), m, runp1);
-  GB_BTRY(cudaGetLastError());
-  GB_BTRY(cub::DeviceScan::InclusiveSum(tmp, scan_bytes, runp1, runp1, (int64_t)m, s));
-  uint32_t np32 = 0;
-  GB_BTRY(cudaMemcpyAsync(&np32, runp1 + (m - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  GB_BTRY(cudaStreamSynchronize(s));
-  const uint64_t npairs = np32;
-  // the cached layout, one allocation (parts 256-byte aligned)
-  auto part = [](uint64_t bytes) { return (bytes + 255) & ~uint64_t(255); };
-  const uint64_t sz_dst = part(2 * mpad), sz_roff = part(mpad), sz_crun = part(4 * nchunks), sz_rsrc = part(4 * npairs),
-                 sz_tasks = part(16 * tasks.size());
-  GB_BTRY(cudaMalloc(&b->mem, sz_dst + sz_roff + sz_crun + sz_rsrc + sz_tasks));
-  char* q = static_cast<char*>(b->mem);
-  b->dst = reinterpret_cast<uint16_t*>(q);
-  q += sz_dst;
-  b->roff = reinterpret_cast<uint8_t*>(q);
-  q += sz_roff;
-  b->crun = reinterpret_cast<uint32_t*>(q);
-  q += sz_crun;
-  b->rsrc = reinterpret_cast<uint32_t*>(q);
-  q += sz_rsrc;
-  b->tasks = reinterpret_cast<uint4*>(q);
-  b->ntasks = (uint32_t)tasks.size();
-  b->npairs = npairs;
-  b->nchunks = nchunks;
-  GB_BTRY(cudaMemsetAsync(b->dst, 0xFF, 2 * mpad, s));  // padding: kBinPad
-  GB_BTRY(cudaMemsetAsync(b->roff, 0, mpad, s));
   GB_BTRY(cudaMemcpyAsync(b->tasks, tasks.data(), 16 * tasks.size(), cudaMemcpyHostToDevice, s));
-  bin_place_kernel<<<grid, 256, 0, s>>>(dk.Current(), dv.Current(), runp1, m, dfirst, dpad, b->dst, b->crun, b->rsrc);
+  GB_BTRY(cudaMemsetAsync(b->crun + nchunks, 0, sizeof(uint32_t), s));
+  bin_place_kernel<<<grid, 256, 0, s>>>(dv.Current(), dfirst, dpad, P, nchunks, b->src, b->flag, b->crun);
   GB_BTRY(cudaGetLastError());
-  bin_roff_kernel<<<grid, 256, 0, s>>>(dk.Current(), runp1, m, dfirst, dpad, b->crun, b->roff);
-  GB_BTRY(cudaGetLastError());
-  bin_chunk_sort_kernel<<<g->sm_count * 16, kBinChunk, 0, s>>>(b->dst, b->roff, nchunks);
+  GB_BTRY(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, b->crun, b->crun, (int64_t)(nchunks + 1), s));
+  uint32_t runs = 0;
+  GB_BTRY(cudaMemcpyAsync(&runs, b->crun + nchunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GB_BTRY(cudaStreamSynchronize(s));
+  GB_BTRY(cudaMalloc(&b->rdst, sizeof(uint32_t) * std::max<uint32_t>(runs, 1)));
+  bin_runs_kernel<<<grid, 256, 0, s>>>(dv.Current(), dfirst, dpad, P, nchunks, b->crun, b->rdst);
   GB_BTRY(cudaGetLastError());
   GB_BTRY(cudaStreamSynchronize(s));
 #undef GB_BTRY
@@ -1411,6 +1509,8 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   const unsigned long long cap = worklists::ring_capacity(2ull * nchunks + g->m / ((uint64_t)t.tile_edges * 32) + 8192);
   size_t need = carve_size<PrCtl>(1) + 5 * carve_size<float>(n) + (out_dev ? 0 : carve_size<float>(n));
   if (kind != PrKind::Pull) need += 2 * carve_size<float>(n);
+  const uint32_t nheavy = g->perm ? std::min(sched.nheavy, kBinHubs) : 0;  // degree order: the first ids
+  need += 2 * carve_size<double>(nheavy);
   if (kind == PrKind::Push) need += 3 * carve_size<uint32_t>(n) + fl.bytes;
   if (kind == PrKind::PushAsync) need += carve_size<char>(worklists::ring_bytes(cap));
   const bool rows = (kind == PrKind::Pull || kind == PrKind::PullResidual) && !g->perm;  // row sweeps in file order
@@ -1437,6 +1537,7 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   a.c[1] = cv.take<float>(n);
   a.acc = cv.take<float>(n);
   a.acc2 = cv.take<float>(n);
+  a.hacc = cv.take<double>(2 * (size_t)nheavy);
   if (kind != PrKind::Pull) {
     a.residual = cv.take<float>(n);
     a.delta = cv.take<float>(n);
@@ -1482,15 +1583,17 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
       // contiguous range)
       if (ensure_pr_bins(g, s) == GB_OK) {
         const PrBins* b = g->prb;
-        a.b_dst = b->dst;
-        a.b_roff = b->roff;
+        a.b_src = b->src;
+        a.b_flag = b->flag;
         a.b_crun = b->crun;
-        a.b_rsrc = b->rsrc;
+        a.b_rdst = b->rdst;
+        a.b_nheavy = nheavy;
+        GB_CUDA(cudaMemsetAsync(a.hacc, 0, sizeof(double) * 2 * nheavy, s));
         a.b_tasks = b->tasks;
         a.b_ntasks = b->ntasks;
         kfn = reinterpret_cast<const void*>(&pr_pull_binned<kBinBlock>);
         block = kBinBlock;
-        smem = sizeof(float) * kBinPart;
+        smem = kBinSmem;
         GB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       } else {
         clear_error();
@@ -1507,15 +1610,17 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
     if (g->perm && (g->order == GB_ORDER_DEGREE || g->order == GB_ORDER_DEGREE_UNSORTED)) {
       if (ensure_pr_bins(g, s) == GB_OK) {  // else the row sweep
         const PrBins* b = g->prb;
-        a.b_dst = b->dst;
-        a.b_roff = b->roff;
+        a.b_src = b->src;
+        a.b_flag = b->flag;
         a.b_crun = b->crun;
-        a.b_rsrc = b->rsrc;
+        a.b_rdst = b->rdst;
+        a.b_nheavy = nheavy;
+        GB_CUDA(cudaMemsetAsync(a.hacc, 0, sizeof(double) * 2 * nheavy, s));
         a.b_tasks = b->tasks;
         a.b_ntasks = b->ntasks;
         kfn = reinterpret_cast<const void*>(&pr_resid_binned<kBinBlock>);
         block = kBinBlock;
-        smem = sizeof(float) * kBinPart;
+        smem = kBinSmem;
         GB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       } else {
         clear_error();

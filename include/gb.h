@@ -330,9 +330,9 @@ int gb_cc(gb_graph* g, int algo, uint32_t* label_out, gb_stats* stats,
  * <= tol or after max_iter iterations.  rank_out[n] float.  On a
  * degree-ordered graph (gb_graph_reorder) this and gb_pagerank_pull_residual
  * run over a binned copy of the arcs built on the first call and kept with
- * the graph until gb_graph_free (about 3 bytes per arc plus 4 per
- * (source, 32 K-destination partition) pair: 1.6 GB at RMAT-24; building it
- * takes 12 bytes per arc of temporary device memory).  Where it cannot be
+ * the graph until gb_graph_free (about 2.2 bytes per arc plus 4 per
+ * (32 K-source block, destination) pair: 1.5 GB at RMAT-24; building it
+ * takes 20 bytes per arc of temporary device memory).  Where it cannot be
  * built the row sweep runs. */
 int gb_pagerank_pull(gb_graph* g, float alpha, float tol, uint32_t max_iter,
                      float* rank_out, uint32_t* iters_out, gb_stats* stats,
