@@ -1154,7 +1154,7 @@ __device__ __forceinline__ void far_file(const SsspArgs& a, uint32_t* farq, uint
 }
 
 // Load a region into shared memory with 16-byte loads: its distances (base
-// is a multiple of kRegion, so 16-byte aligned), its nv + 1 offsets relative
+// is a multiple of kRegion and a.dist 16-byte aligned, see run_sssp_region), its nv + 1 offsets relative
 // to o0, and its na arcs from o0 (any alignment: the unaligned head and tail
 // are loaded one by one).  Only elements inside the arrays are read.
 __device__ __forceinline__ void region_load(const SsspArgs& a, uint32_t base, uint32_t nv, uint64_t o0, uint32_t na,
@@ -1673,8 +1673,8 @@ __global__ void sssp_reach_kernel(const uint32_t* __restrict__ dist, const uint6
 
 }  // namespace
 
-// Error word, statistics and the host copy of the distances after the
-// persistent kernel.
+// Error word, statistics and the copy of the distances to the caller's array
+// after the persistent kernel.
 static int finish_sssp(gb_graph* g, const SsspArgs& a, unsigned long long* reach, const KernelTimer& kt, uint32_t launches,
                 uint32_t* dist_out, bool out_dev, gb_stats* stats, cudaStream_t s) {
   const uint32_t n = g->n;
@@ -1699,10 +1699,8 @@ static int finish_sssp(gb_graph* g, const SsspArgs& a, unsigned long long* reach
     stats->launches = launches;
     stats->kernel_ms = kt.ms();
   }
-  if (!out_dev) {
-    int st = copy_out(dist_out, a.dist, sizeof(uint32_t) * n, s);
-    if (st != GB_OK) return st;
-  }
+  int st = copy_out(dist_out, a.dist, sizeof(uint32_t) * n, s);  // nothing when they are the same array
+  if (st != GB_OK) return st;
   if (stats || !out_dev) {
     GB_CUDA(cudaStreamSynchronize(s));
     if (*pin) return dev_err_status(*pin, "gb_sssp_delta");
@@ -1715,10 +1713,14 @@ static int run_sssp_region(gb_graph* g, uint32_t src, uint32_t shift, uint32_t n
                            uint32_t* dist_out, bool out_dev, gb_stats* stats, cudaStream_t s) {
   const uint32_t n = g->n;
   const uint32_t words = (n + 31) / 32;
+  // the regions' distances are loaded 16 bytes at a time: a device output that
+  // does not start on a 16-byte boundary (a slice of a larger array) gets its
+  // distances from an array of the workspace, copied behind the kernel
+  const bool direct = out_dev && reinterpret_cast<uintptr_t>(dist_out) % 16 == 0;
   // each region is queued at most once at a time
   const unsigned long long cap = worklists::ring_capacity((uint64_t)nregions + 1024);
   const size_t need = carve_size<SsspCtl>(1) + 2 * carve_size<uint32_t>(words) + 2 * carve_size<uint32_t>(n) +
-                      (out_dev ? 0 : carve_size<uint32_t>(n)) + carve_size<unsigned long long>(2) +
+                      (direct ? 0 : carve_size<uint32_t>(n)) + carve_size<unsigned long long>(2) +
                       carve_size<uint32_t>(nregions) + carve_size<char>(worklists::ring_bytes(cap));
   int st = ws_reserve(g, need, s);
   if (st != GB_OK) return st;
@@ -1730,7 +1732,7 @@ static int run_sssp_region(gb_graph* g, uint32_t src, uint32_t shift, uint32_t n
   a.far[0] = cv.take<uint32_t>(n);
   a.far[1] = cv.take<uint32_t>(n);
   unsigned long long* reach = cv.take<unsigned long long>(2);
-  a.dist = out_dev ? dist_out : cv.take<uint32_t>(n);
+  a.dist = direct ? dist_out : cv.take<uint32_t>(n);
   ra.pend = cv.take<uint32_t>(words);
   ra.rq = cv.take<uint32_t>(nregions);
   ra.nregions = nregions;

@@ -256,6 +256,38 @@ def test_sssp_regions_bit_exact(cuda_device, shift):
                     assert (dg.sssp(src, shift) == want).all()
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+def test_sssp_regions_output_at_any_word(cuda_device, offset):
+    """A device output that starts 4, 8, 12 or 16 bytes into an allocation:
+    the region kernel (the default on a grid in file order, and asked for)
+    loads distances 16 bytes at a time.  Graphs of degree 4 and 5 (rows of
+    slots, offsets), several regions and a ragged last one; the words around
+    the output stay as they were."""
+    import torch
+
+    grid = grid2d(70, 61)
+    a = np.repeat(np.arange(grid.n), grid.degrees())
+    v = np.arange(0, grid.n - 62, 500)
+    more = HostCSR.from_edges(grid.n, np.concatenate([a, v, v + 62]), np.concatenate([grid.col, v + 62, v]))
+    assert more.degrees().max() > 4 and grid.degrees().max() == 4
+    for g in (grid, more):
+        assign_weights_u32(g, 1, 255, seed=5)
+        with DeviceGraph(g, symmetric=True) as dg:
+            for mode in (0, 3):
+                dg.set_tuning(sssp_async=mode)
+                for src in (0, g.n - 1):
+                    want = oracle.sssp_dijkstra(g, src)
+                    buf = torch.full((g.n + offset + 4,), -7, dtype=torch.int32, device="cuda")
+                    out = buf[offset:offset + g.n]
+                    dg.sssp(src, 13, out=out)
+                    assert (out.cpu().numpy().view(np.uint32) == want).all()
+                    out.fill_(-7)
+                    _, st = dg.sssp(src, 13, out=out, stats=True)
+                    assert st["pull_rounds"] > 0  # the region kernel
+                    assert (out.cpu().numpy().view(np.uint32) == want).all()
+                    assert (buf[:offset] == -7).all() and (buf[offset + g.n:] == -7).all()
+
+
 def test_sssp_local_queues_rmat(cuda_device):
     g, perm = rmat(14, 16, seed=12, symmetrize=False)
     assign_weights_u32(g, 1, 255, seed=12)
