@@ -236,15 +236,22 @@ __global__ void __launch_bounds__(BLOCK) cc_labelprop(CcArgs a) {
     if (gtid == 0) ctl->rounds = r + 1;
     // a round that hooked nothing leaves every label a root already
     if (*reinterpret_cast<volatile uint32_t*>(changed) == 0) break;
+    // The giant's root may have gone under another.  One thread follows it,
+    // before the barrier (the compression moves no root): the skip is sound
+    // only with one label for every thread, and behind the barrier the next
+    // round's hooks already lower p[giant].
+    if (skip_giant && gtid == 0) {
+      uint32_t x = giant;
+      while (x != a.p[x]) x = a.p[x];
+      ctl->giant = x;
+    }
     compress_all(a, gtid, gthreads);
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-    if (r == 0 && a.half) {
+    if (sampling) {
       if (blockIdx.x == 0) sample_giant<BLOCK>(a, ctl);
       if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
-      giant = *reinterpret_cast<volatile uint32_t*>(&ctl->giant);
-    } else if (a.half) {
-      giant = *reinterpret_cast<volatile uint32_t*>(&a.p[giant]);  // the giant's root may have gone under another
     }
+    if (a.half) giant = *reinterpret_cast<volatile uint32_t*>(&ctl->giant);
   }
   my_scanned = warp_sum(my_scanned);
   if (lane == 0 && my_scanned) atomicAdd(&ctl->scanned, my_scanned);

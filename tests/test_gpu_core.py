@@ -513,6 +513,36 @@ def test_pagerank_row_sweep_edges(cuda_device, n, order):
         assert abs(rst["iterations"] - rit) <= 2
 
 
+@pytest.mark.parametrize("k,n_giant", [(3, 40), (1000, 500), (30000, 20000)])
+def test_cc_giant_goes_under_smaller_roots(cuda_device, k, n_giant):
+    """k triangles whose least ids are below the giant component's hang on it
+    by their third arcs, which the first round does not read: in the second
+    round every triangle hooks the giant's root at once (joins that go on
+    through several labels), so its label falls while the rows are walked.
+    Ids: k triangles' first and second vertices, the head of the giant, the
+    triangles' third vertices, the rest of the giant; rows are sorted, so a
+    row's first two arcs stay inside its triangle or the giant's head."""
+    head = 2 * k
+    third = head + n_giant
+    rest = third + k
+    n = rest + max(n_giant, k)
+    i = np.arange(k)
+    h = np.arange(head, third)
+    g = np.arange(rest, n)
+    rng = np.random.default_rng(k)
+    hang = rng.permutation(g)[:k]  # the giant's end of each triangle's arc
+    a = np.concatenate([i, i, k + i, h[:-1], g, g, third + i])
+    b = np.concatenate([k + i, third + i, third + i, h[1:], head + (g - rest) % n_giant,
+                        head + (g - rest + 1) % n_giant, hang])
+    src, dst = np.concatenate([a, b]), np.concatenate([b, a])
+    order = np.lexsort((dst, src))
+    csr = HostCSR.from_edges(n, src[order], dst[order])
+    for algo in (GB_CC_LABELPROP, GB_CC_AFFOREST):
+        with DeviceGraph(csr, symmetric=True) as dg:
+            for _ in range(5):
+                assert (dg.cc(algo) == 0).all()
+
+
 @pytest.mark.parametrize("method,kw", [("pagerank_pull_residual", {}), ("pagerank_push", {}),
                                        ("pagerank_push", {"algo": "async"})])
 def test_pagerank_residual_converges_to_fixed_point(cuda_device, method, kw):
