@@ -264,6 +264,7 @@ int gb_graph_assign_weights_u32(gb_graph* g, uint32_t lo, uint32_t hi, uint64_t 
   cudaFree(g->ell);  // its rows carry the weights
   g->ell = nullptr;
   g->ell_d = 0;
+  g->region_arcs = 0;
   if (g->m)
     weights_u32_kernel<<<grid_for(g, g->m), 256, 0, s>>>(g->w, g->m, stream_key(seed, kTagWeightU32), lo,
                                                          (uint64_t)hi - lo + 1);
@@ -303,6 +304,7 @@ int gb_graph_assign_weights_reference(gb_graph* g, int min_value, int max_value,
   cudaFree(g->ell);                       // uint32 weights ride in the fixed-width rows
   g->ell = nullptr;
   g->ell_d = 0;
+  g->region_arcs = 0;
   void** dst = edge_bytes == 4 ? reinterpret_cast<void**>(&g->w) : reinterpret_cast<void**>(&g->wf);
   const size_t bytes = 4 * std::max<uint64_t>(g->m, 1);
   if (!*dst) {

@@ -55,6 +55,8 @@ struct gb_graph {
   // fraction of arcs inside their region, for SSSP
   uint64_t region_arcs = 0;
   double region_local = 0.0;
+  bool region_near = false;    // no arc spans more ids than a region has
+  double region_weight = 0.0;  // sum of the uint32 weights
   uint32_t max_degree = 0;
   // all-vertex sweep schedule (sweep.cuh), cached per (heavy, tile)
   uint2* sweep_tiles = nullptr;

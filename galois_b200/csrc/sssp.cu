@@ -1073,13 +1073,16 @@ __device__ __forceinline__ void st_release_cta(uint32_t* p, uint32_t v) {
   cuda::atomic_ref<uint32_t, cuda::thread_scope_block>(*p).store(v, cuda::memory_order_release);
 }
 
-// Largest arc count of any region (out[0], the host check that regions fit)
-// and the number of arcs whose two ends share a region (out[1]).
-__global__ void region_arcs_kernel(const uint64_t* __restrict__ offs, const uint32_t* __restrict__ col, uint32_t n,
-                                   uint32_t nregions, unsigned long long* out) {
+// Largest arc count of any region (out[0], the host check that regions fit),
+// the number of arcs whose two ends share a region (out[1]), the number whose
+// ends are more than a region's width of ids apart (out[2]) and the sum of the
+// weights (out[3]).
+__global__ void region_arcs_kernel(const uint64_t* __restrict__ offs, const uint32_t* __restrict__ col,
+                                   const uint32_t* __restrict__ w, uint32_t n, uint32_t nregions,
+                                   unsigned long long* out) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  unsigned long long mine = 0, local = 0;
+  unsigned long long mine = 0, local = 0, far = 0, weight = 0;
   for (uint64_t r = tid; r < nregions; r += stride) {
     const uint64_t b = r * kRegion, e = b + kRegion < (uint64_t)n ? b + kRegion : (uint64_t)n;
     mine = max(mine, (unsigned long long)(offs[e] - offs[b]));
@@ -1087,15 +1090,24 @@ __global__ void region_arcs_kernel(const uint64_t* __restrict__ offs, const uint
   // arcs by row: a thread per vertex
   for (uint64_t v = tid; v < n; v += stride) {
     const uint64_t r = v / kRegion;
-    for (uint64_t j = offs[v]; j < offs[v + 1]; ++j) local += (uint64_t)col[j] / kRegion == r;
+    for (uint64_t j = offs[v]; j < offs[v + 1]; ++j) {
+      const uint64_t u = col[j];
+      local += u / kRegion == r;
+      far += (u > v ? u - v : v - u) > kRegion;
+      weight += w[j];
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     mine = max(mine, __shfl_xor_sync(kFull, mine, o));
     local += __shfl_xor_sync(kFull, local, o);
+    far += __shfl_xor_sync(kFull, far, o);
+    weight += __shfl_xor_sync(kFull, weight, o);
   }
   if ((threadIdx.x & 31) == 0) {
     atomicMax(out, mine);
     atomicAdd(out + 1, local);
+    atomicAdd(out + 2, far);
+    atomicAdd(out + 3, weight);
   }
 }
 
@@ -1709,10 +1721,10 @@ static int finish_sssp(gb_graph* g, const SsspArgs& a, unsigned long long* reach
 }
 
 // The region kernel (every region's arcs fit in shared memory).
-static int run_sssp_region(gb_graph* g, uint32_t src, uint32_t shift, uint32_t nregions,
-                           uint32_t* dist_out, bool out_dev, gb_stats* stats, cudaStream_t s) {
+static int run_sssp_region(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, bool out_dev, gb_stats* stats, cudaStream_t s) {
   const uint32_t n = g->n;
   const uint32_t words = (n + 31) / 32;
+  const uint32_t nregions = (uint32_t)(((uint64_t)n + kRegion - 1) / kRegion);
   // the regions' distances are loaded 16 bytes at a time: a device output that
   // does not start on a 16-byte boundary (a slice of a larger array) gets its
   // distances from an array of the workspace, copied behind the kernel
@@ -1762,6 +1774,68 @@ static int run_sssp_region(gb_graph* g, uint32_t src, uint32_t shift, uint32_t n
   return finish_sssp(g, a, reach, kt, 2, dist_out, out_dev, stats, s);
 }
 
+// Whether a call relaxes regions in shared memory: asked for (sssp_async 3,
+// whenever every region's arcs fit), or by default on a graph of low degree
+// whose regions fit, where the region kernel is the faster one.
+//  * Numbered by locality: when the regions keep 90 % of the arcs inside
+//    (4096^2 grid: 29.3 against 38.5 ms for the phase-synchronous kernel).
+//  * In file order that depends on the graph's depth in regions and on the
+//    hops that a bucket holds, H = 2^shift / mean weight.  Region / phase-
+//    synchronous time, weights 1..255, shift 13 (H = 64) where not said:
+//    - no arc may span more than a region's width: otherwise few hops cross the
+//      graph and its regions are reloaded for little work each (4000 vertices
+//      of mean degree 3 at random 2.4, 100 communities of 64 with some arcs
+//      between them 1.65, the same of 2048 1.5);
+//    - H >= 12: a bucket is two barriers more for the region kernel (grids of
+//      601 x 433, 2000 x 100, 300 x 1000: H = 2 1.11 / 0.98 / 1.30, unit
+//      weights and H = 8 1.15 / 1.18 / 1.28, H = 16 0.87 / 0.73 / 0.95);
+//    - the regions keep 97 % of the arcs (2000 x 100 0.51, 700 x 120 0.60,
+//      64 x 64 0.33, a path 0.27, 20 000 x 40 0.34; H = 2048 0.43 / 0.66 /
+//      0.29 / 0.17 / 0.33), or 75 % of them when every region has an SM of its
+//      own and H < 96, beyond which a region is settled again and again
+//      (601 x 433, 89 %: H = 64 0.81, 128 0.97, 2048 1.82; 300 x 1000, 76 %:
+//      0.92, 0.97, 1.69; 120 x 700, 83 %: 0.61, 0.63, 1.24; with more regions
+//      than SMs 9000 x 250, 94 %: 0.99, 1.20; below 75 %: 100 x 2000, 51 %:
+//      0.95, 0.95, 3.5; 6000 vertices of mean degree 2 in a band of 2000 ids,
+//      60 %: 1.54).
+static int takes_regions(gb_graph* g, const gb_tuning& t, uint32_t shift, cudaStream_t s, bool* region) {
+  *region = false;
+  const uint32_t n = g->n;
+  const uint32_t nregions = (uint32_t)(((uint64_t)n + kRegion - 1) / kRegion);
+  if (!(t.sssp_async == 3 || (t.sssp_async == 0 && (g->order == GB_ORDER_LOCALITY || t.local_depth > 0)))) return GB_OK;
+  if (!g->region_arcs) {  // once per graph (and after a relabelling or new weights)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GB_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return GB_OK;  // a captured first call cannot wait for the counts
+    const int rst = ws_reserve(g, 256, s);
+    if (rst != GB_OK) return rst;
+    unsigned long long* dout = static_cast<unsigned long long*>(g->ws);
+    unsigned long long* hout = static_cast<unsigned long long*>(g->pinned);
+    GB_CUDA(cudaMemsetAsync(dout, 0, 4 * sizeof(unsigned long long), s));
+    region_arcs_kernel<<<g->sm_count * 8, 256, 0, s>>>(g->offs, g->col, g->w, n, nregions, dout);
+    GB_CUDA(cudaGetLastError());
+    GB_CUDA(cudaMemcpyAsync(hout, dout, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    GB_CUDA(cudaStreamSynchronize(s));
+    g->region_arcs = hout[0] + 1;
+    g->region_local = g->m ? (double)hout[1] / (double)g->m : 1.0;
+    g->region_near = hout[2] == 0;
+    g->region_weight = (double)hout[3];
+  }
+  if (g->region_arcs - 1 > kRegionArcs) return GB_OK;
+  if (t.sssp_async == 3) {
+    *region = true;
+  } else if (g->order == GB_ORDER_LOCALITY) {
+    *region = g->region_local >= 0.9;
+  } else {
+    // H >= 12 and H < 96, without a division by a weight sum of zero
+    const double width = (double)(1ull << shift) * (double)g->m;
+    *region = g->region_near && width >= 12.0 * g->region_weight &&
+              (g->region_local >= 0.97 ||
+               (g->region_local >= 0.75 && nregions <= (uint32_t)g->sm_count && width < 96.0 * g->region_weight));
+  }
+  return GB_OK;
+}
+
 int run_sssp(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, gb_stats* stats,
              cudaStream_t s) {
   if (!g->w) GB_FAIL(GB_ERR_ARG, "gb_sssp_delta: graph has no uint32 edge weights");
@@ -1775,39 +1849,10 @@ int run_sssp(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, gb_s
   // light (entries pack the degree in 16 bits and the begin offset in 48)
   const bool async = t.sssp_async > 0 && local_depth > 0 && g->max_degree <= t.heavy_degree &&
                      g->max_degree < 65536 && g->m < (1ull << 48);
-  // regions in shared memory: asked for (sssp_async 3: whenever every
-  // region's arcs fit), or by default on a bounded-degree graph, whatever its
-  // order, whose regions fit and keep most arcs inside: 90 % of them (measured
-  // on the 4096^2 grid by locality: 29.3 ms against 38.5 ms for the
-  // phase-synchronous kernel; file-order strips of a 1500 x 800 grid, 80 %:
-  // 13.0 against 9.2 ms), or half of them when every region has an SM of its
-  // own and none waits for another (file order, grids of 601 x 433, 89 %:
-  // 2.9 against 3.8 ms; 300 x 1000, 76 %: 4.9 / 5.2; 100 x 2000, 51 %: 8.6 /
-  // 9.2; 64 x 64: 0.12 / 0.38)
   bool region = false;
-  const uint32_t nregions = (uint32_t)(((uint64_t)n + kRegion - 1) / kRegion);
-  if (t.sssp_async == 3 || (t.sssp_async == 0 && (g->order == GB_ORDER_LOCALITY || local_depth > 0))) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    // a captured first call cannot wait for the count: it runs as if it failed
-    if (!g->region_arcs) GB_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (!g->region_arcs && cap == cudaStreamCaptureStatusNone) {  // once per graph (and after a relabelling)
-      int rst = ws_reserve(g, 256, s);
-      if (rst != GB_OK) return rst;
-      unsigned long long* dout = static_cast<unsigned long long*>(g->ws);
-      unsigned long long* hout = static_cast<unsigned long long*>(g->pinned);
-      GB_CUDA(cudaMemsetAsync(dout, 0, 2 * sizeof(unsigned long long), s));
-      region_arcs_kernel<<<g->sm_count * 8, 256, 0, s>>>(g->offs, g->col, n, nregions, dout);
-      GB_CUDA(cudaGetLastError());
-      GB_CUDA(cudaMemcpyAsync(hout, dout, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-      GB_CUDA(cudaStreamSynchronize(s));
-      g->region_arcs = hout[0] + 1;
-      g->region_local = g->m ? (double)hout[1] / (double)g->m : 1.0;
-    }
-    const bool fits = g->region_arcs && g->region_arcs - 1 <= kRegionArcs;
-    const double keep = nregions <= (uint32_t)g->sm_count ? 0.5 : 0.9;
-    region = t.sssp_async == 3 ? fits : fits && g->region_local >= keep;
-  }
-  if (region) return run_sssp_region(g, src, shift, nregions, dist_out, out_dev, stats, s);
+  const int rst = takes_regions(g, t, shift, s, &region);
+  if (rst != GB_OK) return rst;
+  if (region) return run_sssp_region(g, src, shift, dist_out, out_dev, stats, s);
   FrontierLayout fl = frontier_layout(n, g->m, t.heavy_degree, t.tile_edges);
   SweepSched sched{};
   if (!async && g->max_degree > t.heavy_degree) {  // heavy rows of a bitmap frontier come from the tile schedule

@@ -263,10 +263,14 @@ typedef struct gb_tuning {
                             rounds = region visits, pull_rounds =
                             shared-memory rounds;
                             0 = library default: regions on a graph of
-                            low degree (local queues on, or
-                            GB_ORDER_LOCALITY) whose regions fit and keep
-                            >= 90 % of the arcs inside (>= 50 % when there
-                            is an SM for every region), else a grid
+                            low degree whose regions fit, where they are
+                            the faster kernel -- GB_ORDER_LOCALITY: they
+                            keep >= 90 % of the arcs inside; other orders,
+                            with local queues on: no arc spans more than
+                            2048 ids, a bucket is at least 12 mean weights
+                            wide, and they keep >= 97 % of the arcs (or
+                            >= 75 % with an SM for every region and buckets
+                            of less than 96 mean weights) -- else a grid
                             barrier after every phase; < 0 = a grid
                             barrier after every phase */
 } gb_tuning;

@@ -10,7 +10,7 @@ import torch
 import oracle
 from galois_b200 import (GB_CC_AFFOREST, GB_CC_LABELPROP, GB_CC_UNIONFIND, GB_ORDER_DEGREE,
                          GB_ORDER_DEGREE_UNSORTED, GB_ORDER_NONE, DeviceGraph, GbError, HostCSR,
-                         assign_weights_f32, assign_weights_u32, grid2d, rmat)
+                         assign_weights_f32, assign_weights_u32, erdos_renyi, grid2d, rmat)
 from galois_b200 import _lib
 from galois_b200._lib import GB_ORDER_LOCALITY
 from galois_b200.graph import pack_graphs
@@ -247,20 +247,47 @@ def test_auto_order_and_default_region_kernel(cuda_device):
                 dg.set_tuning(sssp_async=0)
 
 
-@pytest.mark.parametrize("rows,cols,shuffled", [(1, 2047, False), (1, 2048, False), (33, 65, False), (90, 433, False),
-                                                (601, 433, False), (100, 2900, False), (90, 433, True)])
-def test_default_region_rule_in_file_order(cuda_device, rows, cols, shuffled):
+@pytest.mark.parametrize("rows,cols,shift,region", [
+    (1, 2047, 13, True), (1, 2048, 13, True), (33, 65, 13, True), (90, 433, 13, True), (601, 433, 13, True),
+    (90, 433, 8, False), (90, 433, 14, False), (700, 120, 8, False), (700, 120, 11, True), (700, 120, 20, True),
+    (100, 2000, 13, False), (100, 2900, 13, False)])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_default_region_rule_in_file_order(cuda_device, rows, cols, shift, region, shuffled):
     """A grid in file order takes the region kernel when its regions of 2048
-    ids keep at least half of the arcs and each has an SM; with its ids
-    shuffled it does not.  Same distances either way, from the first vertex,
-    the middle and the last."""
+    ids keep most of the arcs, no arc spans more ids than that and a bucket
+    holds enough hops, and not too many where the regions keep fewer; with the
+    ids shuffled only a graph of one region does.  Same distances either way,
+    from the first vertex, the middle and the last."""
     g = grid2d(rows, cols)
     if shuffled:
         perm = np.random.default_rng(1).permutation(g.n)
         g = HostCSR.from_edges(g.n, perm[np.repeat(np.arange(g.n), g.degrees())], perm[g.col])
+        region = region and g.n <= 2048
     assign_weights_u32(g, 1, 255, seed=rows)
     with DeviceGraph(g, symmetric=True) as dg:
         for src in (0, g.n // 2, g.n - 1):
-            got, st = dg.sssp(src, 13, stats=True)
+            got, st = dg.sssp(src, shift, stats=True)
             assert (got == oracle.sssp_dijkstra(g, src)).all()
-            assert (st["pull_rounds"] > 0) == (not shuffled)
+            assert (st["pull_rounds"] > 0) == region
+
+
+def test_default_region_rule_other_graphs(cuda_device):
+    """Small random graphs of two regions keep the phase-synchronous kernel,
+    and the rule follows new weights: unit weights make a bucket of 2^13 too
+    many hops for a grid of which 89 % of the arcs stay inside."""
+    er = erdos_renyi(4000, 3.0, seed=2)
+    assign_weights_u32(er, 1, 255, seed=2)
+    with DeviceGraph(er, symmetric=True) as dg:
+        got, st = dg.sssp(7, 13, stats=True)
+        assert (got == oracle.sssp_dijkstra(er, 7)).all() and st["pull_rounds"] == 0
+    g = grid2d(90, 433)
+    assign_weights_u32(g, 1, 255, seed=4)
+    with DeviceGraph(g, symmetric=True) as dg:
+        assert dg.sssp(0, 13, stats=True)[1]["pull_rounds"] > 0
+        for hi, shift, region in ((1, 13, False), (1, 5, True), (255, 13, True)):
+            dg.assign_weights_u32(1, hi, 9)
+            g.w_u32 = None
+            assign_weights_u32(g, 1, hi, seed=9)
+            got, st = dg.sssp(0, shift, stats=True)
+            assert (got == oracle.sssp_dijkstra(g, 0)).all()
+            assert (st["pull_rounds"] > 0) == region
