@@ -27,6 +27,7 @@
 
 #include "device_common.cuh"
 #include "device_graph.cuh"
+#include "sweep.cuh"
 #include "union_find.cuh"
 
 namespace gb {
@@ -103,12 +104,28 @@ __global__ void mg_roots(const uint32_t* __restrict__ level, uint32_t n, const u
 }
 
 // Union-find over the arcs of the unreached vertices (their neighbours are
-// unreached too: the graphs are symmetric, so each edge is taken once).
+// unreached too: the graphs are symmetric, so each edge is taken once): tasks
+// of 32 consecutive rows, then the heavy rows' tiles, so that no warp walks
+// the row of an unreached hub alone (the call on one graph of 1 M vertices
+// whose unreached component is a star: 10.9 ms by a warp per row, 0.086 with
+// tiles; eight of 100 K 1.12 / 0.083).
 __global__ void mg_link(const uint32_t* __restrict__ level, const uint64_t* __restrict__ offs,
-                        const uint32_t* __restrict__ col, uint32_t n, uint32_t* p) {
+                        const uint32_t* __restrict__ col, uint32_t n, SweepSched sched, uint32_t* p) {
   const uint64_t gwarp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t c = gwarp; c < ((uint64_t)n + 31) >> 5; c += nwarps) {
+  const uint64_t nchunks = ((uint64_t)n + 31) >> 5;
+  for (uint64_t c = gwarp; c < nchunks + sched.ntiles; c += nwarps) {
+    if (c >= nchunks) {
+      const uint2 tv = sched.tiles[c - nchunks];
+      if (level[tv.x] != kInf) continue;
+      const uint64_t vb = ldg(offs + tv.x), ve = ldg(offs + tv.x + 1);
+      const uint64_t b = vb + (uint64_t)tv.y * sched.tile, e = min(ve, b + sched.tile);
+      for (uint64_t j = b + lane_id(); j < e; j += 32) {
+        const uint32_t u = ldg(col + j);
+        if (u < tv.x) link(p, tv.x, u);
+      }
+      continue;
+    }
     const uint64_t v = (c << 5) + lane_id();
     const bool mine = v < n && level[v] == kInf;
     if (!__any_sync(kFull, mine)) continue;
@@ -116,7 +133,8 @@ __global__ void mg_link(const uint32_t* __restrict__ level, const uint64_t* __re
     uint32_t d = 0;
     if (mine) {
       b = ldg(offs + v);
-      d = (uint32_t)(ldg(offs + v + 1) - b);
+      const uint64_t dd = ldg(offs + v + 1) - b;
+      d = dd > sched.heavy ? 0u : (uint32_t)dd;
     }
     warp_expand(b, d, (uint32_t)v, [&](bool on, uint64_t e, uint32_t, uint32_t x) {
       if (!on) return;
@@ -144,6 +162,20 @@ __global__ void mg_label(const uint32_t* __restrict__ level, uint32_t n, const u
 
 // CC labels of every graph from its BFS levels (see the file comment).
 int cc_from_levels(gb_graph* g, const uint32_t* d_level, uint32_t ng, uint32_t* d_label, cudaStream_t s) {
+  // the heavy rows' tiles, when some row needs them (built once per graph; a
+  // call that is captured before that was done walks every row by a warp)
+  const gb_tuning t = effective_tuning(g);
+  SweepSched sched{};
+  sched.heavy = 0xFFFFFFFFu;
+  if (g->max_degree > t.heavy_degree) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool built = g->sweep_tiles && g->sweep_heavy == t.heavy_degree && g->sweep_tile == t.tile_edges;
+    if (!built) GB_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+      const int rc = ensure_sweep_schedule(g, t.heavy_degree, t.tile_edges, s, &sched);
+      if (rc != GB_OK) return rc;
+    }
+  }
   // after the BFS: its workspace is free again, and holds two queues of n ids
   const size_t need = carve_size<uint32_t>(ng) + carve_size<uint32_t>(g->n);
   int st = ws_reserve(g, need, s);
@@ -154,7 +186,7 @@ int cc_from_levels(gb_graph* g, const uint32_t* d_level, uint32_t ng, uint32_t* 
   GB_CUDA(cudaMemsetAsync(root, 0xFF, sizeof(uint32_t) * ng, s));
   const int blocks = g->sm_count * 8;
   mg_roots<<<blocks, 256, 0, s>>>(d_level, g->n, g->mg_first, ng, root, p);
-  mg_link<<<blocks, 256, 0, s>>>(d_level, g->offs, g->col, g->n, p);
+  mg_link<<<blocks, 256, 0, s>>>(d_level, g->offs, g->col, g->n, sched, p);
   mg_label<<<blocks, 256, 0, s>>>(d_level, g->n, g->mg_first, ng, root, p, d_label);
   GB_CUDA(cudaGetLastError());
   return GB_OK;

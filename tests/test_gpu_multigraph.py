@@ -56,6 +56,45 @@ def test_multigraph_labels_from_levels(cuda_device, sizes):
             assert np.array_equal(lv, want_lv) and np.array_equal(lb, want_lb)
 
 
+@pytest.mark.parametrize("hub_at", [2, 700, 40000])
+@pytest.mark.parametrize("heavy,tile", [(0, 0), (16, 32)])
+def test_multigraph_unreached_hubs(cuda_device, hub_at, heavy, tile):
+    """Sources in small components beside unreached ones with hubs of many
+    tiles (most neighbours' ids above the hub's, some, or none), rows of
+    exactly the heavy degree, a graph whose hub is reached, and a captured
+    call."""
+    import torch
+
+    n = 40001
+    arcs = [(0, 1)] + [(hub_at, v) for v in range(2, n) if v != hub_at and v % 7]
+    arcs += [(v, v + 7) for v in range(7, n - 700, 7)][:5000]
+    arcs += [(3, v) for v in range(8, 8 + 7 * 16, 7) if v != hub_at]  # a row of 17 or so
+    src, dst = np.array(arcs + [(b, a) for a, b in arcs]).T
+    order = np.lexsort((dst, src))
+    hub = HostCSR.from_edges(n, src[order], dst[order])
+    reached = HostCSR.from_edges(900, [0] * 899 + list(range(1, 900)), list(range(1, 900)) + [0] * 899)
+    graphs = [hub, reached, erdos_renyi(50, 2.0, seed=1), hub]
+    packed, first = pack_graphs(graphs)
+    local = np.array([0, 5, 0, 1], np.uint32)
+    want_lv, want_lb = expected(graphs, local)
+    with DeviceGraph(packed, symmetric=True) as dg:
+        if heavy:
+            dg.set_tuning(heavy_degree=heavy, tile_edges=tile)
+        lv, lb = dg.multi_graph_bfs_cc(first, local)
+        assert np.array_equal(lv, want_lv) and np.array_equal(lb, want_lb)
+        d_lv = torch.zeros(packed.n, dtype=torch.int32, device="cuda")
+        d_lb = torch.zeros(packed.n, dtype=torch.int32, device="cuda")
+        dg.multi_graph_bfs_cc(first, local, level_out=d_lv, label_out=d_lb)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            dg.multi_graph_bfs_cc(first, local, level_out=d_lv, label_out=d_lb)
+        d_lv.fill_(-1), d_lb.fill_(-1)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(d_lv.cpu().numpy().view(np.uint32), want_lv)
+        assert np.array_equal(d_lb.cpu().numpy().view(np.uint32), want_lb)
+
+
 def test_multigraph_rejects_crossing_arcs_and_bad_sources(cuda_device):
     graphs = make_graphs(4, seed=1)
     packed, first = pack_graphs(graphs)
