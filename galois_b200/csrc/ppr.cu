@@ -62,11 +62,21 @@ uint32_t ppr_tile(const gb_graph* g) {
   return t;
 }
 
+// Tiles whose partial rows one warp adds up, one after another.  A longer row
+// is added up in two passes, span by span and then the spans' sums, with a grid
+// barrier between; graphs without such a row do neither.  Forward + adjoint of a
+// star of 500 K vertices, B = 4 / 128, ms: 135 / 315 with one warp for all 15 625
+// tiles, 29 / 50 so; eight hubs of 62 K arcs 34 / 75, 22 / 43.  Spans of 128
+// tiles took 20 / 41 there, but their pass and barrier cost RMAT-18, whose
+// longest row has some 400, 3 to 6 %.
+constexpr uint32_t kPprSpan = 512;
+
 struct RowSched {
   uint2* tiles = nullptr;
   uint32_t* heavy = nullptr;
   uint32_t ntiles = 0, nheavy = 0;
   uint32_t tile = 0;  // arcs per tile; a row of more is heavy
+  bool spans = false;  // some row has more than kPprSpan tiles
 };
 
 struct PprState {
@@ -199,7 +209,7 @@ struct Wide {
   static constexpr int U = 8 / G > 2 ? 8 / G : 2;
 };
 
-// Sum over arcs [b, e) of wn * x[col] for this lane's 4 columns; `first` holds
+// Sum over arcs [b, e) of wn * x[col] for this lane's 4 columns; `m` holds
 // the row's first 32 arcs.  Every group of LPA lanes returns the whole sum.
 template <int LPA, int U>
 __device__ __forceinline__ float4 row_sum(const IterArgs& a, const float* __restrict__ x, uint64_t b, uint64_t e,
@@ -328,6 +338,16 @@ __global__ void __launch_bounds__(kPprBlock, MINB) ppr_iterate(IterArgs a) {
       return act ? *reinterpret_cast<const float4*>(x + (uint64_t)r * a.B + 4 * lane)
                  : make_float4(0.f, 0.f, 0.f, 0.f);
     };
+    // this lane's columns of `cnt` partial rows, `step` tiles apart from tile t, in
+    // order; stored in tile t's slot if asked
+    auto sum_tiles = [&](uint64_t t, uint32_t cnt, uint32_t step, bool store) {
+      float4* h = reinterpret_cast<float4*>(a.part + t * a.B) + lane;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+      for (uint32_t k = 0; k < cnt; ++k) acc = f4_fma(1.f, h[(uint64_t)k * step * (a.B / 4)], acc);
+      if (store) *h = acc;
+      return acc;
+    };
     for (uint64_t t = gwarp; t < ntasks; t += nwarps) {
       if (t < a.sched.ntiles) {  // one tile of a heavy row
         const uint2 tv = a.sched.tiles[t];
@@ -382,6 +402,18 @@ __global__ void __launch_bounds__(kPprBlock, MINB) ppr_iterate(IterArgs a) {
       }
     }
     if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
+    // rows of more than kPprSpan tiles: each span's sum, in tile order, into
+    // its first tile's slot
+    if (WIDE && a.sched.spans) {  // uniform
+      for (uint64_t t = gwarp; t < a.sched.ntiles; t += nwarps) {
+        const uint2 tv = a.sched.tiles[t];
+        if (tv.y % kPprSpan != 0) continue;
+        const uint64_t d = ldg(a.offs + tv.x + 1) - ldg(a.offs + tv.x);
+        const uint32_t cnt = (uint32_t)((d + tile - 1) / tile);
+        if (cnt > kPprSpan && act) sum_tiles(t, min(kPprSpan, cnt - tv.y), 1, true);
+      }
+      if (!grid_barrier(&ctl->bar, gridDim.x, &ctl->err, deadline)) return;
+    }
     // heavy rows: their tiles follow one another from the one with k = 0
     for (uint64_t t = gwarp; t < a.sched.ntiles; t += nwarps) {
       const uint2 tv = a.sched.tiles[t];
@@ -391,10 +423,8 @@ __global__ void __launch_bounds__(kPprBlock, MINB) ppr_iterate(IterArgs a) {
       if constexpr (WIDE) {
         if (!act) continue;
         const float4 o = old_row(tv.x);
-        const float4* h = reinterpret_cast<const float4*>(a.part + t * a.B) + lane;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (uint32_t k = 0; k < cnt; ++k) acc = f4_fma(1.f, h[(uint64_t)k * (a.B / 4)], acc);
+        const float4 acc = cnt > kPprSpan ? sum_tiles(t, (cnt + kPprSpan - 1) / kPprSpan, kPprSpan, false)
+                                          : sum_tiles(t, cnt, 1, false);
         finish(tv.x, acc, o);
       } else {
         float acc = 0.f;
@@ -558,6 +588,12 @@ const void* grad_kernel(uint32_t B) {
   }
 }
 
+// *any = 1 if some row has more than kPprSpan tiles.
+__global__ void ppr_any_span(const uint2* __restrict__ tiles, uint32_t ntiles, uint32_t* any) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
+    if (tiles[t].y == kPprSpan) *any = 1;
+}
+
 // out[c] = sum_r |src[r][c]| for the B columns of a vertex-major [n][B] array.
 __global__ void ppr_colnorm(const float* __restrict__ src, uint32_t n, uint32_t B, double* out) {
   __shared__ double s_sum[128];
@@ -607,6 +643,16 @@ int ensure_state(gb_graph* g, cudaStream_t s, PprState** out) {
     GB_CUDA(cudaMalloc(&st->flags, sizeof(uint32_t) * ((n + 31) / 32)));
     GB_CUDA(cudaMalloc(&st->l1, sizeof(double) * 4 * 128));
     GB_CUDA(cudaMalloc(&st->colnorm, sizeof(double) * 128));
+    uint32_t* any = reinterpret_cast<uint32_t*>(st->l1);  // scratch until the first solve
+    uint32_t* h_any = static_cast<uint32_t*>(g->pinned);
+    GB_CUDA(cudaMemsetAsync(any, 0, 2 * sizeof(uint32_t), s));
+    ppr_any_span<<<g->sm_count, 256, 0, s>>>(st->fwd.tiles, st->fwd.ntiles, any);
+    ppr_any_span<<<g->sm_count, 256, 0, s>>>(st->bwd.tiles, st->bwd.ntiles, any + 1);
+    GB_CUDA(cudaGetLastError());
+    GB_CUDA(cudaMemcpyAsync(h_any, any, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    GB_CUDA(cudaStreamSynchronize(s));
+    st->fwd.spans = h_any[0] != 0;
+    st->bwd.spans = h_any[1] != 0;
   }
   *out = static_cast<PprState*>(g->ppr_state);
   return GB_OK;

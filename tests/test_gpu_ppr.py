@@ -99,6 +99,46 @@ def test_row_and_tile_edges(cuda_device, B):
     assert rel(gw, gw_ref) < 1e-3
 
 
+@pytest.mark.parametrize("B", [1, 4, 20, 128])
+def test_hub_spans(cuda_device, B):
+    """Hubs of exactly 512 tiles of 32 arcs, one arc more, 1024 tiles and one
+    arc more (512 tiles make a span, added up before the spans' sums are), in
+    both directions, beside light rows; two runs give the same bits."""
+    import torch
+
+    from galois_b200.ppr import ppr
+
+    rng = np.random.default_rng(5)
+    n, src, dst = 33001, [], []
+    for j, d in enumerate((16384, 16385, 32768, 32769)):
+        to = rng.choice(np.arange(4, n), d, replace=False)
+        src += [np.full(d, j), to]
+        dst += [to, np.full(d, j)]
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    g = HostCSR.from_edges(n, src, dst)
+    assert g.m < 148 * 32 * 16 * 64  # tiles of 32 arcs
+    assign_weights_f32(g, seed=6)
+    T = rng.random((n, B)).astype(np.float32) * (rng.random((n, B)) < 0.1)
+    T /= np.maximum(T.sum(0), 1e-30)
+    c = rng.standard_normal((n, B)).astype(np.float32)
+    w64 = g.w_f32.astype(np.float64)
+    x_ref = oppr.forward(g, T.astype(np.float64), w64, ALPHA)
+    gT_ref, gw_ref = oppr.backward(g, x_ref, c.astype(np.float64), w64, ALPHA)
+    runs = []
+    with DeviceGraph(g) as dg:
+        for _ in range(2):
+            Tt = torch.from_numpy(T).cuda().requires_grad_(True)
+            w = torch.from_numpy(g.w_f32).cuda().requires_grad_(True)
+            x = ppr(dg, Tt, w, ALPHA, 1e-7)
+            runs.append((x, *torch.autograd.grad((torch.from_numpy(c).cuda() * x).sum(), (Tt, w))))
+    for a, b in zip(*runs):
+        assert torch.equal(a, b)
+    x, gT, gw = (t.detach().cpu().numpy() for t in runs[0])
+    assert np.allclose(x, x_ref, atol=1e-6, rtol=1e-4)
+    assert rel(gT, gT_ref) < 1e-3
+    assert rel(gw, gw_ref) < 1e-3
+
+
 def test_heavy_rows_tiled(cuda_device):
     import torch
 
