@@ -210,7 +210,7 @@ struct Wide {
 };
 
 // Sum over arcs [b, e) of wn * x[col] for this lane's 4 columns; `m` holds
-// the row's first 32 arcs.  Every group of LPA lanes returns the whole sum.
+// the row's first 32 arcs.  The first LPA lanes return the whole sum.
 template <int LPA, int U>
 __device__ __forceinline__ float4 row_sum(const IterArgs& a, const float* __restrict__ x, uint64_t b, uint64_t e,
                                           ArcLoad m) {
@@ -239,8 +239,11 @@ __device__ __forceinline__ float4 row_sum(const IterArgs& a, const float* __rest
     }
     m = nm;
   }
+  // lanes past a short row's arcs hold zeros: no step for them
+  const uint32_t lanes = e - b < 32 / LPA ? (uint32_t)(e - b) * LPA : 32u;
 #pragma unroll
   for (int o = LPA; o < 32; o <<= 1) {
+    if (o >= lanes) break;  // uniform
     acc.x += __shfl_xor_sync(kFull, acc.x, o);
     acc.y += __shfl_xor_sync(kFull, acc.y, o);
     acc.z += __shfl_xor_sync(kFull, acc.z, o);
@@ -285,11 +288,17 @@ __device__ __forceinline__ void ppr_rows(const uint64_t* __restrict__ offs, cons
   }
 }
 
-// Rows per task: 32, or fewer when there are too few rows for every warp.
+// Rows per task: 32, or fewer when there are too few rows for every warp; then
+// half as many if that leaves fewer rows on the longest warp's path (a task's
+// start, its offsets and then its first row's arcs, counted as two rows).  A
+// 300 x 300 grid had 19 rows a warp in tasks of 16, so 32 for some: forward +
+// adjoint, B = 4 / 128, 6.2 / 10.2 ms, now 4.9 / 8.2; 100 K vertices of mean
+// degree 3 6.1 / 11.2, 4.8 / 9.2.
 __device__ __forceinline__ uint32_t ppr_rows_per_task(uint32_t n, uint64_t nwarps) {
   uint32_t r = 32;
   while (r > 1 && (uint64_t)n < nwarps * r) r >>= 1;
-  return r;
+  auto path = [&](uint32_t rows) { return ((uint64_t)n / rows + nwarps) / nwarps * (rows + 2); };
+  return r >= 8 && path(r / 2) < path(r) ? r / 2 : r;
 }
 
 // LPA: lanes per row of B floats; 0 for B = 1 (lanes over arcs).

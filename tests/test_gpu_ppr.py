@@ -99,6 +99,32 @@ def test_row_and_tile_edges(cuda_device, B):
     assert rel(gw, gw_ref) < 1e-3
 
 
+@pytest.mark.parametrize("rows,cols", [(97, 31), (300, 257), (401, 500)])
+@pytest.mark.parametrize("B", [4, 8, 128])
+def test_grid_rows_per_task(cuda_device, rows, cols, B):
+    """Rows of two to four arcs, for which a row's sum takes fewer steps over
+    the lanes, and vertex counts that give a task 1, 8 and 16 rows, ragged at
+    the end: the forward solve against 64 bits, and each column's sum, which it
+    keeps."""
+    import torch
+
+    from galois_b200 import grid2d
+    from galois_b200.ppr import ppr
+
+    g = grid2d(rows, cols)
+    assign_weights_f32(g, seed=3)
+    rng = np.random.default_rng(rows)
+    T = np.zeros((g.n, B), np.float32)
+    T[rng.integers(0, g.n, 8 * B), np.tile(np.arange(B), 8)] = 0.125
+    x_ref = oppr.forward(g, T.astype(np.float64), g.w_f32.astype(np.float64), ALPHA)
+    with DeviceGraph(g) as dg:
+        w = torch.from_numpy(g.w_f32).cuda()
+        x = ppr(dg, torch.from_numpy(T).cuda(), w, ALPHA, 1e-7)
+        # every vertex has out-arcs, so the solve keeps each column's sum
+        assert np.allclose(x.double().sum(0).cpu().numpy(), T.astype(np.float64).sum(0), rtol=1e-5)
+    assert np.allclose(x.cpu().numpy(), x_ref, atol=1e-6, rtol=1e-4)
+
+
 @pytest.mark.parametrize("B", [1, 4, 20, 128])
 def test_hub_spans(cuda_device, B):
     """Hubs of exactly 512 tiles of 32 arcs, one arc more, 1024 tiles and one
