@@ -36,8 +36,7 @@ struct GridBar {
   unsigned int count;  // grid_barrier_last
   unsigned int gen;
   unsigned int word;  // grid_barrier: its top bit flips when every CTA has arrived
-};  // the kernel's error word follows (grid_barrier reads both with one load)
-static_assert(sizeof(GridBar) == 12, "GridBar and the error word behind it fill 16 bytes");
+};
 
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
@@ -63,17 +62,22 @@ __device__ __forceinline__ uint64_t kernel_deadline() { return globaltimer_ns() 
 // Grid-wide barrier for a cooperative launch of `nblocks` CTAs (1-D grid).
 // Returns false (for every thread of the CTA) if the error word is set, the
 // wait exceeded `timeout_ns`, or the kernel passed `deadline`; callers then
-// leave the kernel.  `bar` is 16-byte aligned and `err` the word behind it.
+// leave the kernel.
 //
 // What bounds it is the chain of L2 round trips, so a barrier is one atomic
-// and the polls of the same word: the CTAs of a phase add up to 2^31 (CTA 0
-// adds 2^31 - (nblocks - 1), the others 1), so the top bit flips with the last
-// arrival and the low bits are zero again.  The error word comes with each
-// poll (one 8-byte load: an error raised before any CTA's arrival is seen by
-// whoever sees the flip).  The arrival is a release and the fence after the
-// polls the matching acquire.  Measured on B200 against the count, the generation read before it
-// and the release store after it: 148 CTAs 2.4 -> 1.3 us, 592 3.1 -> 1.5 us,
-// 1184 4.2 -> 2.6 us, without the error read that was one more round trip.
+// and the polls of the same word, encoded as in the CUDA toolkit's own grid
+// sync (cooperative_groups/details/sync.h): the CTAs of a phase add up to 2^31
+// (CTA 0 adds 2^31 - (nblocks - 1), the others 1), so the top bit flips with
+// the last arrival and the low bits are zero again.  The arrival is a release
+// and a poll that sees the flip, with the fence behind it, the acquire: both
+// 4-byte accesses of one word.  The error word is read with the first poll and
+// with every 32nd after it.  So a CTA may leave a barrier without an error that
+// another raised shortly before; the next barrier sees it, and the kernels bound
+// every queue count they read.
+// Measured on B200, 256 threads a CTA, against a count, the generation read
+// before it and the release store after it, then the error read: 148 CTAs 2.69
+// -> 1.36 us, 592 3.54 -> 1.66, 1184 5.09 -> 3.81 (polls of word and error with
+// one 8-byte load: 1.38, 2.42, 4.4; two loads with every poll: 1.42, 3.25, 6.8).
 __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nblocks, int* err,
                                              uint64_t deadline = ~0ull,
                                              uint64_t timeout_ns = 2000000000ull) {
@@ -82,26 +86,31 @@ __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nblocks, int
   if (threadIdx.x == 0) {
     if (blockIdx.x == 0 && globaltimer_ns() > deadline) raise_err(err, kDevTimeout);
     const unsigned add = blockIdx.x == 0 ? 0x80000000u - (nblocks - 1) : 1u;
-    unsigned old;
-    unsigned long long now;  // the word, and the error word above it
+    unsigned old, now;
+    int failed = 0;
     asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
                  : "=r"(old)
                  : "l"(__cvta_generic_to_global(&bar->word)), "r"(add)
                  : "memory");
     int ok = 1;
     uint64_t t0 = 0;
-    for (unsigned spins = 1;; ++spins) {
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];"
-                   : "=l"(now)
+    for (unsigned spins = 0;; ++spins) {
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
+                   : "=r"(now)
                    : "l"(__cvta_generic_to_global(&bar->word))
                    : "memory");
-      if (now >> 32) {
+      if ((spins & 31u) == 0)
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
+                     : "=r"(failed)
+                     : "l"(__cvta_generic_to_global(err))
+                     : "memory");
+      if (failed) {
         ok = 0;
         break;
       }
-      if (((unsigned)now ^ old) >> 31) break;
+      if ((now ^ old) >> 31) break;
       __nanosleep(20);
-      if ((spins & 31u) == 0) {
+      if ((spins & 31u) == 31u) {
         const uint64_t t = globaltimer_ns();
         if (!t0) t0 = t;
         if (t - t0 > timeout_ns) {

@@ -51,7 +51,7 @@ extern "C" int gb_probe_bounded_waits(int which, uint32_t limit_us, void* stream
   GB_CUDA(cudaMalloc(&mem, bytes));
   GB_CUDA(cudaMemsetAsync(mem, 0, bytes, s));
   GridBar* bar = reinterpret_cast<GridBar*>(mem);
-  int* err = reinterpret_cast<int*>(bar + 1);  // where grid_barrier reads it
+  int* err = reinterpret_cast<int*>(mem + 64);
   worklists::Ring ring = worklists::ring_layout(mem + 256, cap);
   const uint64_t limit_ns = (uint64_t)limit_us * 1000ull;
   cudaError_t e = cudaSuccess;
