@@ -98,8 +98,8 @@ constexpr uint32_t kStage = 128;
 // Queue a warp's n staged vertices: their degrees are read together, the light
 // ones go to light queue qb and the heavy ones' tiles to tile queue qb, both
 // reserved with one 64-bit atomic.  Adds the lane's share of the vertices and
-// of their degrees to items / deg.  `limit`: a degree sum above which nothing
-// is queued -- the next level then pulls, and reads the bitmap (the top hubs
+// of their degrees to items / deg.  `limit`: a degree sum times alpha above
+// which nothing is queued -- the next level then pulls, and reads the bitmap (the top hubs
 // of RMAT-20 have 40 K tiles, which one warp wrote and nobody read; a search
 // from one of them 191 -> 154 us).
 // All lanes call.
@@ -127,12 +127,18 @@ __device__ __noinline__ void bfs_drain(const BfsArgs& a, const uint32_t* slots, 
     lights += __popc(lm[k]);
   }
   __syncwarp();  // the slots may be refilled
-  if ((double)warp_sum(deg) > limit) return;
+  // A lane's share is clipped so that the sum stays in 32 bits: at worst a queue
+  // is written that nobody reads.  One reduction, no division and no scan
+  // without tiles: a level with a small frontier lasts as long as this chain
+  // (1000 x 1000 grid, 2000 levels: 16.9 -> 16.3 ms, a path 7.6 -> 7.3 us a level).
+  if ((double)__reduce_add_sync(kFull, (uint32_t)min(deg, 1ull << 26)) * a.alpha > limit) return;
   uint32_t incl = tiles;
+  if (__any_sync(kFull, tiles != 0)) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(kFull, incl, o);
-    if ((int)lane >= o) incl += t;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, incl, o);
+      if ((int)lane >= o) incl += t;
+    }
   }
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   unsigned long long base = 0;
@@ -208,7 +214,7 @@ __global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(const __grid_constant
     const int prev_pull = pull;
     if (can_pull) {
       if (!pull) {
-        if ((double)scout > (double)edges_to_check / a.alpha) { pull = 1; old_items = 0; }
+        if ((double)scout * a.alpha > (double)edges_to_check) { pull = 1; old_items = 0; }
       } else {
         if (!(items >= old_items || items > a.n / a.beta)) pull = 0;
       }
@@ -262,8 +268,8 @@ __global__ void __launch_bounds__(BLOCK, 4) bfs_persistent(const __grid_constant
       // cheaper barrier; most steps discover something).
       uint32_t staged = 0, q_items = 0;
       unsigned long long q_deg = 0;
-      // the next level pulls when its degree sum is above this (the rule above)
-      const double limit = can_pull ? (double)edges_to_check / a.alpha : CUDART_INF;
+      // the next level pulls when its degree sum times alpha is above this (the rule above)
+      const double limit = can_pull ? (double)edges_to_check : CUDART_INF;
       auto drain = [&]() {
         bfs_drain(a, slots, staged, (L + 1) & 1, &nxt, limit, q_items, q_deg);
         staged = 0;

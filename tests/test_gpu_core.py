@@ -150,6 +150,33 @@ def test_bfs_parent_small_shapes_and_device_output(cuda_device):
         assert e.value.status == _lib.GB_ERR_ARG
 
 
+@pytest.mark.parametrize("alpha", [1e-3, 2.0, 15.0, 1e6])
+@pytest.mark.parametrize("heavy,tile", [(16, 32), (0, 0)])
+def test_bfs_queue_edges(cuda_device, alpha, heavy, tile):
+    """Levels whose vertices have rows of 0 to `heavy` + 1 arcs and of 8, 9 and
+    many tiles side by side (a lane writes up to 8 tiles of its own, the warp
+    the longer runs), with direction switch points at which every warp queues
+    its part of the next level, some do, or none does."""
+    rng = np.random.default_rng(7)
+    n, hubs = 30000, 300
+    deg = rng.integers(0, 40, hubs)
+    deg[:12] = [0, 1, 15, 16, 17, 32, 33, 8 * 32, 8 * 32 + 1, 9 * 32, 40 * 32, 9000]
+    rng.shuffle(deg)
+    src = np.repeat(np.arange(1, hubs + 1), deg)
+    dst = rng.integers(hubs + 1, n, len(src))
+    more = rng.integers(hubs + 1, n, (2, n))  # the levels after them
+    a = np.concatenate([np.zeros(hubs, np.int64), src, more[0]])
+    b = np.concatenate([np.arange(1, hubs + 1), dst, more[1]])
+    g = HostCSR.from_edges(n, np.concatenate([a, b]), np.concatenate([b, a]))
+    for order in (0, 1):
+        with DeviceGraph(g, symmetric=True, reorder=order) as dg:
+            dg.set_tuning(do_alpha=alpha, heavy_degree=heavy, tile_edges=tile)
+            for s in (0, 5, n - 1):
+                want = oracle.bfs_serial(g, s)
+                for _ in range(2):
+                    assert (dg.bfs(s) == want).all(), (order, s)
+
+
 # ---- SSSP ---------------------------------------------------------------------
 
 @pytest.mark.parametrize("shift", [0, 5, 13, 31])
