@@ -355,6 +355,25 @@ def test_cc_min_labels(cuda_device, algo):
         assert (got == want).all()
 
 
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("arcs_per_row", [0.5, 1.24, 1.25, 1.26, 2.0])
+def test_cc_sparse_first_round(cuda_device, arcs_per_row, order):
+    """Symmetric graphs on both sides of 1.25 arcs per row, from which on the
+    first round takes two arcs a row: a hub of many tiles, small components
+    and isolated vertices."""
+    n, hub = 40000, 9000
+    rng = np.random.default_rng(3)
+    edges = int(n * arcs_per_row / 2)
+    a = np.concatenate([np.full(hub, 77), rng.integers(n // 3, n, edges - hub)])
+    b = np.concatenate([rng.permutation(n // 3)[:hub], rng.integers(n // 3, n, edges - hub)])
+    g = HostCSR.from_edges(n, np.concatenate([a, b]), np.concatenate([b, a]))
+    assert abs(g.m - arcs_per_row * n) <= 2
+    want = oracle.cc_union_find(g)
+    with DeviceGraph(g, symmetric=True, reorder=order) as dg:
+        for _ in range(3):
+            assert (dg.cc(GB_CC_LABELPROP) == want).all()
+
+
 def test_cc_directed_is_weak(cuda_device):
     g, _ = rmat(12, 4, seed=5, symmetrize=False)
     sym = HostCSR.from_edges(g.n, np.concatenate([np.repeat(np.arange(g.n), g.degrees()), g.col]),
