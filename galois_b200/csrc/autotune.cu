@@ -25,6 +25,7 @@ namespace gb {
 int run_bfs(gb_graph* g, uint32_t src, uint32_t* level_out, gb_stats* stats, cudaStream_t s, void* scratch,
             size_t scratch_bytes);
 int run_sssp(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, gb_stats* stats, cudaStream_t s);
+int sssp_takes_regions(gb_graph* g, const gb_tuning& t, uint32_t shift, cudaStream_t s, bool* region);
 int run_cc(gb_graph* g, int algo, uint32_t* label_out, gb_stats* stats, cudaStream_t s);
 
 namespace {
@@ -108,6 +109,8 @@ extern "C" int gb_autotune(gb_graph* g, const char* kernel, uint32_t src, const 
   // candidate grid
   std::vector<gb_tuning> cands;
   const gb_tuning base = g->tuning;
+  constexpr uint32_t kSsspShift = 13;  // the sssp program's default bucket width
+  bool region_listed = false;
   for (uint32_t heavy : {32u, 128u, 512u})
     for (uint32_t tile : {128u, 256u, 512u}) {
       if (tile < heavy / 2) continue;
@@ -117,17 +120,23 @@ extern "C" int gb_autotune(gb_graph* g, const char* kernel, uint32_t src, const 
       if (k == "sssp") {
         for (int depth : {-1, 2, 8, 16}) {
           t.local_depth = depth;
+          // the default: where it takes the regions, which use neither the
+          // queues nor the tiles, once, and the phase-synchronous kernel as -1
           t.sssp_async = 0;
-          cands.push_back(t);
+          bool region = false;
+          const int rc = sssp_takes_regions(g, t, kSsspShift, s, &region);
+          if (rc != GB_OK) return rc;
+          if (!region || !region_listed) cands.push_back(t);
+          if (region) {
+            region_listed = true;
+            t.sssp_async = -1;
+            cands.push_back(t);
+          }
           if (depth > 0) {  // asynchronous buckets (taken only when every vertex is light),
             t.sssp_async = 1;  // then over fixed-width rows (degree <= 8)
             cands.push_back(t);
             t.sssp_async = 2;
             cands.push_back(t);
-            if (g->order == GB_ORDER_LOCALITY) {  // 0 took the regions: also without them
-              t.sssp_async = -1;
-              cands.push_back(t);
-            }
           }
         }
       } else if (k == "bfs") {
@@ -150,7 +159,7 @@ extern "C" int gb_autotune(gb_graph* g, const char* kernel, uint32_t src, const 
     for (int rep = 0; rep < 3 && rc == GB_OK; ++rep) {  // first run warms workspaces
       gb_stats st{};
       if (k == "bfs") rc = run_bfs(g, src, out, &st, s, nullptr, 0);
-      else if (k == "sssp") rc = run_sssp(g, src, 13, out, &st, s);
+      else if (k == "sssp") rc = run_sssp(g, src, kSsspShift, out, &st, s);
       else if (k == "cc") rc = run_cc(g, GB_CC_LABELPROP, out, &st, s);
       else rc = gb_pagerank_pull(g, 0.85f, 1e-6f, 1000, reinterpret_cast<float*>(out), nullptr, &st, s);
       if (rc == GB_ERR_NOT_CONVERGED) rc = GB_OK;

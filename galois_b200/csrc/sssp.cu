@@ -1798,7 +1798,7 @@ static int run_sssp_region(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* 
 //      than SMs 9000 x 250, 94 %: 0.99, 1.20; below 75 %: 100 x 2000, 51 %:
 //      0.95, 0.95, 3.5; 6000 vertices of mean degree 2 in a band of 2000 ids,
 //      60 %: 1.54).
-static int takes_regions(gb_graph* g, const gb_tuning& t, uint32_t shift, cudaStream_t s, bool* region) {
+int sssp_takes_regions(gb_graph* g, const gb_tuning& t, uint32_t shift, cudaStream_t s, bool* region) {
   *region = false;
   const uint32_t n = g->n;
   const uint32_t nregions = (uint32_t)(((uint64_t)n + kRegion - 1) / kRegion);
@@ -1850,7 +1850,7 @@ int run_sssp(gb_graph* g, uint32_t src, uint32_t shift, uint32_t* dist_out, gb_s
   const bool async = t.sssp_async > 0 && local_depth > 0 && g->max_degree <= t.heavy_degree &&
                      g->max_degree < 65536 && g->m < (1ull << 48);
   bool region = false;
-  const int rst = takes_regions(g, t, shift, s, &region);
+  const int rst = sssp_takes_regions(g, t, shift, s, &region);
   if (rst != GB_OK) return rst;
   if (region) return run_sssp_region(g, src, shift, dist_out, out_dev, stats, s);
   FrontierLayout fl = frontier_layout(n, g->m, t.heavy_degree, t.tile_edges);

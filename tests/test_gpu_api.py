@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from galois_b200 import DeviceGraph, assign_weights_u32, rmat, write_gr
+from galois_b200 import DeviceGraph, HostCSR, _lib, assign_weights_u32, grid2d, rmat, write_gr
 
 pytestmark = pytest.mark.gpu
 
@@ -74,6 +74,33 @@ def test_load_gr_and_autotune(cuda_device, gr_files, tmp_path):
         assert (dg.cc() == oracle.cc_union_find(g)).all()
     finally:
         dg.free()
+
+
+@pytest.mark.parametrize("order", [0, _lib.GB_ORDER_LOCALITY])
+@pytest.mark.parametrize("rows,cols,isolated", [(90, 433, False), (60, 50, True), (100, 2000, False)])
+def test_autotune_sssp_times_both_defaults(cuda_device, rows, cols, isolated, order):
+    """On grids that take the region kernel by default (and one that does not)
+    the tuned SSSP is about as fast as the phase-synchronous kernel at any
+    depth it tries and as the default, and exact.  From an isolated vertex the
+    region kernel is the slower one."""
+    g = grid2d(rows, cols)
+    src = 0
+    if isolated:
+        g = HostCSR(np.append(g.end_offs, g.m), g.col)
+        src = g.n - 1
+    assign_weights_u32(g, 1, 255, seed=2)
+    want = oracle.sssp_dijkstra(g, src)
+
+    def ms(dg, **kw):
+        dg.set_tuning(**kw)
+        assert (dg.sssp(src, 13) == want).all()
+        return min(dg.sssp(src, 13, stats=True)[1]["kernel_ms"] for _ in range(5))
+
+    with DeviceGraph(g, symmetric=True, reorder=order) as dg:
+        others = [ms(dg, sssp_async=0)] + [ms(dg, sssp_async=-1, local_depth=d) for d in (2, 8, 16)]
+        dg.set_tuning(sssp_async=0, local_depth=0)
+        dg.autotune("sssp", src, None)
+        assert ms(dg) <= 1.5 * min(others) + 0.01
 
 
 def test_pool_reuses_blocks_and_trims(cuda_device):

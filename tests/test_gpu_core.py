@@ -193,14 +193,17 @@ def test_sssp_rmat_directed_bit_exact(cuda_device, shift):
 
 @pytest.mark.parametrize("local_depth,block", [(-1, 256), (8, 256), (64, 1024)])
 def test_sssp_grid_many_buckets(cuda_device, local_depth, block):
+    """The phase-synchronous kernel (sssp_async = -1: the default would take
+    regions for the widest buckets) without local queues, with queues and
+    with large blocks."""
     g = grid2d(96, 80)
     assign_weights_u32(g, 1, 255, seed=3)
     want = oracle.sssp_dijkstra(g, 0)
     with DeviceGraph(g, symmetric=True) as dg:
-        dg.set_tuning(local_depth=local_depth, block_threads=block)
+        dg.set_tuning(local_depth=local_depth, block_threads=block, sssp_async=-1)
         for shift in (13, 8, 3):
             got, st = dg.sssp(0, shift, stats=True)
-            assert (got == want).all()
+            assert (got == want).all() and st["pull_rounds"] == 0
             if shift <= 8:
                 assert st["buckets"] > 10
 
@@ -229,8 +232,9 @@ def test_sssp_async_buckets_bit_exact(cuda_device, shift):
                     got, st = dg.sssp(src, shift, stats=True)
                     assert (got == want).all(), f"async {mode} n={g.n} src={src}"
                     assert st["vertices_reached"] == int((want != INF).sum())
-                dg.set_tuning(sssp_async=0)
-                assert (dg.sssp(src, shift) == want).all(), f"phase-synchronous n={g.n} src={src}"
+                dg.set_tuning(sssp_async=-1)
+                got, st = dg.sssp(src, shift, stats=True)
+                assert (got == want).all() and st["pull_rounds"] == 0, f"phase-synchronous n={g.n} src={src}"
 
 
 def test_sssp_async_small_ring_and_blocks(cuda_device):
