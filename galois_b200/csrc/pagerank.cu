@@ -1271,9 +1271,6 @@ int hot_scratch(gb_graph* g, cudaStream_t s, size_t* bytes, size_t* sort_bytes) 
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   GB_CUDA(cudaStreamIsCapturing(s, &cap));
   if (cap != cudaStreamCaptureStatusNone) return GB_OK;
-  size_t free_bytes = 0, total_bytes = 0;
-  GB_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-  if (sizeof(uint32_t) * (g->m + g->n) > free_bytes / 4) return GB_OK;
   cub::DoubleBuffer<uint32_t> key(nullptr, nullptr), id(nullptr, nullptr);
   GB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, *sort_bytes, key, id, (int64_t)g->n, 0, 32, s));
   *bytes = carve_size<unsigned long long>(1) + 4 * carve_size<uint32_t>(g->n) + carve_size<char>(*sort_bytes);
@@ -1303,15 +1300,26 @@ int ensure_hot(gb_graph* g, size_t sort_bytes, cudaStream_t s) {
   GB_CUDA(cudaMemcpyAsync(harcs, arcs, sizeof(*arcs), cudaMemcpyDeviceToHost, s));
   GB_CUDA(cudaStreamSynchronize(s));
   if ((double)*harcs < kHotShare * (double)m) return GB_OK;
-  if (cudaMalloc(&h->col, sizeof(uint32_t) * (m + n)) != cudaSuccess) {
+  // asked here, once per graph that qualifies: the question alone takes up to
+  // 10 ms on a device whose memory is nearly all in use
+  size_t free_bytes = 0, total_bytes = 0;
+  GB_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (sizeof(uint32_t) * (m + n) > free_bytes / 4) return GB_OK;
+  uint32_t* cols = nullptr;
+  if (cudaMalloc(&cols, sizeof(uint32_t) * (m + n)) != cudaSuccess) {
     cudaGetLastError();
-    h->col = nullptr;
     return GB_OK;
   }
-  h->rank = h->col + m;
-  hot_rank_kernel<<<grid, 256, 0, s>>>(id.Current(), n, h->rank);
-  hot_col_kernel<<<grid, 256, 0, s>>>(g->col, m, h->rank, h->col);
-  GB_CUDA(cudaGetLastError());
+  uint32_t* const rank = cols + m;
+  hot_rank_kernel<<<grid, 256, 0, s>>>(id.Current(), n, rank);
+  hot_col_kernel<<<grid, 256, 0, s>>>(g->col, m, rank, cols);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {  // the handle must not be left with columns that nothing wrote
+    cudaFree(cols);
+    return cuda_fail(e, "pagerank: renamed columns");
+  }
+  h->col = cols;
+  h->rank = rank;
   return GB_OK;
 }
 
@@ -1523,6 +1531,7 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
   if (st != GB_OK && hot > need) {
     clear_error();
     hot = 0;
+    g->prh = new (std::nothrow) PrHot;  // the columns stay: not tried again on every call
     st = ws_reserve(g, need, s);
   }
   if (st != GB_OK) return st;

@@ -337,7 +337,11 @@ int gb_cc(gb_graph* g, int algo, uint32_t* label_out, gb_stats* stats,
  * the graph until gb_graph_free (about 2.2 bytes per arc plus 4 per
  * (32 K-source block, destination) pair: 1.5 GB at RMAT-24; building it
  * takes 20 bytes per arc of temporary device memory).  Where it cannot be
- * built the row sweep runs. */
+ * built the row sweep runs.  In file order, when a few vertices take at least a
+ * quarter of the arcs (power-law graphs of more than 49 152 vertices), both keep
+ * a copy of the columns renamed by in-degree with the graph instead: 4 bytes per
+ * arc and per vertex, made on the first call outside stream capture if that is
+ * at most a quarter of the free device memory then, until gb_graph_free. */
 int gb_pagerank_pull(gb_graph* g, float alpha, float tol, uint32_t max_iter,
                      float* rank_out, uint32_t* iters_out, gb_stats* stats,
                      void* stream);
