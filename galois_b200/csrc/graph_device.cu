@@ -266,12 +266,24 @@ int ensure_transpose(gb_graph* g, cudaStream_t stream) {
     cudaFree(indeg);
     cudaFree(tmp);
   };
+  // built whole or not at all: a later call takes t_offs as the sign of all four
+  auto drop = [&]() {
+    cudaFree(g->t_offs);
+    cudaFree(g->t_col);
+    cudaFree(g->t_emap);
+    cudaFree(g->t_wf);
+    g->t_offs = nullptr;
+    g->t_col = nullptr;
+    g->t_emap = nullptr;
+    g->t_wf = nullptr;
+  };
 #define GB_TRY(call)                       \
   do {                                     \
     cudaError_t _e = (call);               \
     if (_e != cudaSuccess) {               \
       st = cuda_fail(_e, #call);           \
       cleanup();                           \
+      drop();                              \
       return st;                           \
     }                                      \
   } while (0)
