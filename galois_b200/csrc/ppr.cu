@@ -626,6 +626,38 @@ __global__ void ppr_scale(const float* __restrict__ src, float scale, uint64_t c
   for (uint64_t i = tid; i < count; i += stride) dst[i] = scale * src[i];
 }
 
+int build_state(gb_graph* g, PprState* st, cudaStream_t s) {
+  const uint32_t n = g->n;
+  const uint64_t m = g->m;
+  const uint32_t tile = ppr_tile(g);
+  st->fwd.tile = st->bwd.tile = tile;
+  int rc = build_row_schedule(g->t_offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->fwd.tiles,
+                              &st->fwd.heavy, &st->fwd.ntiles, &st->fwd.nheavy);
+  if (rc != GB_OK) return rc;
+  rc = build_row_schedule(g->offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->bwd.tiles,
+                          &st->bwd.heavy, &st->bwd.ntiles, &st->bwd.nheavy);
+  if (rc != GB_OK) return rc;
+  const size_t ntiles = std::max<size_t>(1, std::max(st->fwd.ntiles, st->bwd.ntiles));
+  GB_CUDA(cudaMalloc(&st->part, sizeof(float) * 128 * ntiles));
+  GB_CUDA(cudaMalloc(&st->s, sizeof(float) * n));
+  GB_CUDA(cudaMalloc(&st->wn, sizeof(float) * std::max<uint64_t>(m, 1)));
+  GB_CUDA(cudaMalloc(&st->wn_t, sizeof(float) * std::max<uint64_t>(m, 1)));
+  GB_CUDA(cudaMalloc(&st->flags, sizeof(uint32_t) * ((n + 31) / 32)));
+  GB_CUDA(cudaMalloc(&st->l1, sizeof(double) * 4 * 128));
+  GB_CUDA(cudaMalloc(&st->colnorm, sizeof(double) * 128));
+  uint32_t* any = reinterpret_cast<uint32_t*>(st->l1);  // scratch until the first solve
+  uint32_t* h_any = static_cast<uint32_t*>(g->pinned);
+  GB_CUDA(cudaMemsetAsync(any, 0, 2 * sizeof(uint32_t), s));
+  ppr_any_span<<<g->sm_count, 256, 0, s>>>(st->fwd.tiles, st->fwd.ntiles, any);
+  ppr_any_span<<<g->sm_count, 256, 0, s>>>(st->bwd.tiles, st->bwd.ntiles, any + 1);
+  GB_CUDA(cudaGetLastError());
+  GB_CUDA(cudaMemcpyAsync(h_any, any, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  GB_CUDA(cudaStreamSynchronize(s));
+  st->fwd.spans = h_any[0] != 0;
+  st->bwd.spans = h_any[1] != 0;
+  return GB_OK;
+}
+
 int ensure_state(gb_graph* g, cudaStream_t s, PprState** out) {
   int rc = ensure_transpose(g, s);
   if (rc != GB_OK) return rc;
@@ -634,34 +666,11 @@ int ensure_state(gb_graph* g, cudaStream_t s, PprState** out) {
     if (!st) GB_FAIL(GB_ERR_OOM, "ppr: host allocation failed");
     g->ppr_state = st;
     g->ppr_free = free_state;
-    const uint32_t n = g->n;
-    const uint64_t m = g->m;
-    const uint32_t tile = ppr_tile(g);
-    st->fwd.tile = st->bwd.tile = tile;
-    rc = build_row_schedule(g->t_offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->fwd.tiles,
-                            &st->fwd.heavy, &st->fwd.ntiles, &st->fwd.nheavy);
-    if (rc != GB_OK) return rc;
-    rc = build_row_schedule(g->offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->bwd.tiles,
-                            &st->bwd.heavy, &st->bwd.ntiles, &st->bwd.nheavy);
-    if (rc != GB_OK) return rc;
-    const size_t ntiles = std::max<size_t>(1, std::max(st->fwd.ntiles, st->bwd.ntiles));
-    GB_CUDA(cudaMalloc(&st->part, sizeof(float) * 128 * ntiles));
-    GB_CUDA(cudaMalloc(&st->s, sizeof(float) * n));
-    GB_CUDA(cudaMalloc(&st->wn, sizeof(float) * std::max<uint64_t>(m, 1)));
-    GB_CUDA(cudaMalloc(&st->wn_t, sizeof(float) * std::max<uint64_t>(m, 1)));
-    GB_CUDA(cudaMalloc(&st->flags, sizeof(uint32_t) * ((n + 31) / 32)));
-    GB_CUDA(cudaMalloc(&st->l1, sizeof(double) * 4 * 128));
-    GB_CUDA(cudaMalloc(&st->colnorm, sizeof(double) * 128));
-    uint32_t* any = reinterpret_cast<uint32_t*>(st->l1);  // scratch until the first solve
-    uint32_t* h_any = static_cast<uint32_t*>(g->pinned);
-    GB_CUDA(cudaMemsetAsync(any, 0, 2 * sizeof(uint32_t), s));
-    ppr_any_span<<<g->sm_count, 256, 0, s>>>(st->fwd.tiles, st->fwd.ntiles, any);
-    ppr_any_span<<<g->sm_count, 256, 0, s>>>(st->bwd.tiles, st->bwd.ntiles, any + 1);
-    GB_CUDA(cudaGetLastError());
-    GB_CUDA(cudaMemcpyAsync(h_any, any, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GB_CUDA(cudaStreamSynchronize(s));
-    st->fwd.spans = h_any[0] != 0;
-    st->bwd.spans = h_any[1] != 0;
+    rc = build_state(g, st, s);
+    if (rc != GB_OK) {  // whole or not at all: a later call may find the memory
+      free_state(g);
+      return rc;
+    }
   }
   *out = static_cast<PprState*>(g->ppr_state);
   return GB_OK;

@@ -259,3 +259,50 @@ def test_ppr_sharded_single_rank_matches_autograd(cuda_device):
         assert abs(float(loss) - float(lr.detach())) <= 1e-5 * max(1.0, abs(float(lr.detach())))
     finally:
         dist.destroy_process_group()
+
+
+def test_no_memory_then_memory(cuda_device):
+    """First calls on a device without memory for the transpose, then for the
+    solve's own arrays, fail and leave nothing half-made: the next calls fail
+    the same way, and with memory again the result is another handle's."""
+    import torch
+
+    from galois_b200 import _lib, erdos_renyi
+    from galois_b200.ppr import ppr
+
+    g = erdos_renyi(400000, 8.0, seed=3)
+    assign_weights_f32(g, seed=4)
+    T = torch.rand((g.n, 4), device="cuda") / g.n
+    x = torch.empty_like(T)
+    with DeviceGraph(g) as dg:
+        want = ppr(dg, T, None, ALPHA, 1e-6)
+    _lib.check(_lib.lib.gb_pool_trim(), "gb_pool_trim")
+
+    def call(dg):
+        return _lib.lib.gb_ppr_forward(dg.handle, 4, T.data_ptr(), None, ALPHA, 1e-6, 1000, x.data_ptr(), None, None,
+                                       None)
+
+    def take_all():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        held = []
+        for mb in (8192, 1024, 128, 16, 2):
+            while torch.cuda.mem_get_info()[0] > (mb + 4) << 20:
+                try:
+                    held.append(torch.empty(mb << 20, dtype=torch.uint8, device="cuda"))
+                except torch.OutOfMemoryError:
+                    break
+        return held
+
+    for transposed in (False, True):
+        with DeviceGraph(g) as dg:
+            if transposed:
+                dg.build_transpose()
+            held = take_all()
+            for _ in range(2):
+                assert call(dg) == _lib.GB_ERR_OOM
+            del held
+            torch.cuda.empty_cache()
+            assert call(dg) == _lib.GB_OK
+            torch.cuda.synchronize()
+            assert torch.allclose(x, want, atol=1e-9, rtol=1e-5)
