@@ -740,6 +740,13 @@ int solve(gb_graph* g, PprState* st, bool adjoint, uint32_t B, const float* src,
   return GB_OK;
 }
 
+// Rows of several columns are read and written 16 bytes at a time.
+int check_aligned(uint32_t B, const float* p, const char* what) {
+  if (B > 1 && reinterpret_cast<uintptr_t>(p) % 16 != 0)
+    GB_FAIL(GB_ERR_ARG, "ppr: %s must start on a 16-byte boundary (B > 1)", what);
+  return GB_OK;
+}
+
 int check_common(gb_graph* g, uint32_t B, float alpha, uint32_t max_iter) {
   // teleport / rank / arc-weight arrays are indexed by the caller's ids and arcs
   if (g->perm) GB_FAIL(GB_ERR_UNSUPPORTED, "ppr: graph was relabelled; PPR needs file order");
@@ -763,6 +770,8 @@ extern "C" int gb_ppr_forward(gb_graph* g, uint32_t B, const float* teleport, co
   if (rc != GB_OK) return rc;
   GB_CUDA(cudaSetDevice(g->device));
   if (!is_device_ptr(teleport) || !is_device_ptr(x_out)) GB_FAIL(GB_ERR_ARG, "gb_ppr_forward: arrays must be device memory");
+  if ((rc = check_aligned(B, teleport, "teleport")) != GB_OK) return rc;
+  if ((rc = check_aligned(B, x_out, "x_out")) != GB_OK) return rc;
   PprState* st = nullptr;
   if ((rc = ensure_state(g, s, &st)) != GB_OK) return rc;
   if ((rc = prepare_weights(g, st, w, s)) != GB_OK) return rc;
@@ -805,6 +814,8 @@ extern "C" int gb_ppr_backward(gb_graph* g, uint32_t B, const float* x, const fl
   if (!is_device_ptr(x) || !is_device_ptr(gx) || (grad_teleport && !is_device_ptr(grad_teleport)) ||
       (grad_w && !is_device_ptr(grad_w)))
     GB_FAIL(GB_ERR_ARG, "gb_ppr_backward: arrays must be device memory");
+  if ((rc = check_aligned(B, x, "x")) != GB_OK) return rc;
+  if ((rc = check_aligned(B, gx, "gx")) != GB_OK) return rc;
   PprState* st = nullptr;
   if ((rc = ensure_state(g, s, &st)) != GB_OK) return rc;
   if ((rc = prepare_weights(g, st, w, s)) != GB_OK) return rc;

@@ -27,13 +27,19 @@ def _stream(t: torch.Tensor):
     return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """t, or a copy of it where it does not start on a 16-byte boundary (a
+    slice of a larger tensor): the kernels read rows 16 bytes at a time."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class PersonalizedPageRank(torch.autograd.Function):
     @staticmethod
     def forward(ctx, graph: DeviceGraph, teleport: torch.Tensor, w: torch.Tensor | None, alpha: float, tol: float,
                 max_iter: int):
         if not teleport.is_cuda or teleport.dtype != torch.float32:
             raise TypeError("teleport must be a CUDA float32 tensor [n, B]")
-        teleport = teleport.contiguous()
+        teleport = _aligned(teleport.contiguous())
         n, B = teleport.shape
         if n != graph.n:
             raise ValueError(f"teleport has {n} rows, graph has {graph.n} vertices")
@@ -58,7 +64,7 @@ class PersonalizedPageRank(torch.autograd.Function):
     def backward(ctx, gx: torch.Tensor):
         x, w = ctx.saved_tensors
         alpha, tol, max_iter = ctx.params
-        gx = gx.contiguous().to(torch.float32)
+        gx = _aligned(gx.contiguous().to(torch.float32))
         n, B = x.shape
         grad_t = torch.empty_like(x) if ctx.needs_input_grad[1] else None
         grad_w = torch.empty(ctx.graph.m, dtype=torch.float32, device=x.device) if (

@@ -408,7 +408,8 @@ int gb_multi_graph_bfs_cc(gb_graph* g, const uint32_t* graph_first,
  *   teleport: dense [n][B] row-major float, device memory
  *   w:        [m] device floats, or NULL for the uploaded w_f32
  *   x_out:    [n][B] row-major float, device memory
- * The transpose is built on first use. */
+ * With B > 1 teleport and x_out (x and gx below) start on 16-byte boundaries
+ * (else GB_ERR_ARG).  The transpose is built on first use. */
 int gb_ppr_forward(gb_graph* g, uint32_t B, const float* teleport,
                    const float* w, float alpha, float tol, uint32_t max_iter,
                    float* x_out, uint32_t* iters_out, gb_stats* stats,

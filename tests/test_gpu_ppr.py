@@ -306,3 +306,51 @@ def test_no_memory_then_memory(cuda_device):
             assert call(dg) == _lib.GB_OK
             torch.cuda.synchronize()
             assert torch.allclose(x, want, atol=1e-9, rtol=1e-5)
+
+
+@pytest.mark.parametrize("B", [1, 4, 128])
+def test_inputs_at_any_word(cuda_device, B):
+    """Teleport and loss-gradient tensors that start 4 to 12 bytes into an
+    allocation: the autograd entry point copies them, the C entry points
+    refuse what the kernels cannot read 16 bytes at a time."""
+    import torch
+
+    from galois_b200 import _lib
+    from galois_b200.ppr import ppr
+
+    g, T, c = setup(B=4)
+    n = g.n
+    T = torch.from_numpy(np.tile(T, (1, 32))[:, :B].copy()).cuda()
+    c = torch.from_numpy(np.tile(c, (1, 32))[:, :B].copy()).cuda()
+    w = torch.from_numpy(g.w_f32).cuda()
+
+    def at(t, words):
+        buf = torch.empty(t.numel() + words, device="cuda")
+        buf[words:] = t.flatten()
+        return buf[words:].view(t.shape)
+
+    with DeviceGraph(g) as dg:
+        runs = []
+        for words in (0, 1, 2, 3):
+            Tt, wt = at(T, words).requires_grad_(True), w.clone().requires_grad_(True)
+            assert Tt.data_ptr() % 16 == 4 * words
+            x = ppr(dg, Tt, wt, ALPHA, 1e-7)
+            runs.append((x, *torch.autograd.grad(x, (Tt, wt), grad_outputs=at(c, words))))
+        for r in runs[1:]:
+            assert all(torch.equal(a, b) for a, b in zip(r, runs[0]))
+        x = torch.empty((n, B), device="cuda")
+        gw = torch.empty(g.m, device="cuda")
+        ok = _lib.GB_OK if B == 1 else _lib.GB_ERR_ARG
+
+        def forward(t, out):
+            return _lib.lib.gb_ppr_forward(dg.handle, B, t.data_ptr(), None, ALPHA, 1e-7, 1000, out.data_ptr(), None,
+                                           None, None)
+
+        def backward(xs, gx):
+            return _lib.lib.gb_ppr_backward(dg.handle, B, xs.data_ptr(), gx.data_ptr(), None, ALPHA, 1e-7, 1000, None,
+                                            gw.data_ptr(), None, None, None)
+
+        assert forward(T, x) == _lib.GB_OK and backward(x, c) == _lib.GB_OK
+        assert forward(at(T, 1), x) == ok and forward(T, at(x, 3)) == ok
+        assert backward(at(x, 2), c) == ok and backward(x, at(c, 1)) == ok
+        torch.cuda.synchronize()
