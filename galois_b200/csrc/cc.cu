@@ -57,7 +57,6 @@ struct CcArgs {
   uint32_t* p;
   SweepSched sched;
   CcCtl* ctl;
-  uint32_t* hist;  // Afforest root histogram sample
   uint32_t max_rounds;
 };
 
@@ -328,13 +327,12 @@ int run_cc(gb_graph* g, int algo, uint32_t* label_out, gb_stats* stats, cudaStre
   SweepSched sched;
   int st = ensure_sweep_schedule(g, t.heavy_degree, t.tile_edges, s, &sched);
   if (st != GB_OK) return st;
-  const size_t need = carve_size<CcCtl>(1) + carve_size<uint32_t>(1024) + (out_dev ? 0 : carve_size<uint32_t>(n));
+  const size_t need = carve_size<CcCtl>(1) + (out_dev ? 0 : carve_size<uint32_t>(n));
   st = ws_reserve(g, need, s);
   if (st != GB_OK) return st;
   Carver cv(g->ws);
   CcArgs a{};
   a.ctl = cv.take<CcCtl>(1);
-  a.hist = cv.take<uint32_t>(1024);
   a.p = out_dev ? label_out : cv.take<uint32_t>(n);
   a.offs = g->offs;
   a.col = g->col;

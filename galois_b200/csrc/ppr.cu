@@ -73,8 +73,7 @@ constexpr uint32_t kPprSpan = 512;
 
 struct RowSched {
   uint2* tiles = nullptr;
-  uint32_t* heavy = nullptr;
-  uint32_t ntiles = 0, nheavy = 0;
+  uint32_t ntiles = 0;
   uint32_t tile = 0;  // arcs per tile; a row of more is heavy
   bool spans = false;  // some row has more than kPprSpan tiles
 };
@@ -93,10 +92,7 @@ struct PprState {
 void free_state(gb_graph* g) {
   PprState* st = static_cast<PprState*>(g->ppr_state);
   if (!st) return;
-  for (RowSched* r : {&st->fwd, &st->bwd}) {
-    cudaFree(r->tiles);
-    cudaFree(r->heavy);
-  }
+  for (RowSched* r : {&st->fwd, &st->bwd}) cudaFree(r->tiles);
   cudaFree(st->s);
   cudaFree(st->wn);
   cudaFree(st->wn_t);
@@ -631,12 +627,13 @@ int build_state(gb_graph* g, PprState* st, cudaStream_t s) {
   const uint64_t m = g->m;
   const uint32_t tile = ppr_tile(g);
   st->fwd.tile = st->bwd.tile = tile;
-  int rc = build_row_schedule(g->t_offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->fwd.tiles,
-                              &st->fwd.heavy, &st->fwd.ntiles, &st->fwd.nheavy);
-  if (rc != GB_OK) return rc;
-  rc = build_row_schedule(g->offs, n, m, tile, tile, g->sm_count, g->pinned, s, &st->bwd.tiles,
-                          &st->bwd.heavy, &st->bwd.ntiles, &st->bwd.nheavy);
-  if (rc != GB_OK) return rc;
+  for (RowSched* r : {&st->fwd, &st->bwd}) {
+    uint32_t *heavy = nullptr, nheavy = 0;  // not needed: a heavy row is the tiles behind its first one
+    const int rc = build_row_schedule(r == &st->fwd ? g->t_offs : g->offs, n, m, tile, tile, g->sm_count, g->pinned, s,
+                                      &r->tiles, &heavy, &r->ntiles, &nheavy);
+    cudaFree(heavy);
+    if (rc != GB_OK) return rc;
+  }
   const size_t ntiles = std::max<size_t>(1, std::max(st->fwd.ntiles, st->bwd.ntiles));
   GB_CUDA(cudaMalloc(&st->part, sizeof(float) * 128 * ntiles));
   GB_CUDA(cudaMalloc(&st->s, sizeof(float) * n));
