@@ -16,8 +16,8 @@
 //     least id, no arc is read for it, and union-find (larger root under the
 //     smaller) runs over the arcs of the unreached vertices only.  512
 //     Erdos-Renyi graphs of 1 K - 200 K vertices, mean degree 8: union-find
-//     over every arc took 4.1 of 5.8 ms; the call now takes 1.7 ms.  A call for the labels alone runs
-//     union-find over all arcs.
+//     over every arc took 4.1 of 5.5 ms; the call now takes 1.5 ms.  A call
+//     for the labels alone runs union-find over all arcs.
 // After the first call on a layout (validation, buffer set-up) the call
 // issues only stream-ordered work when the outputs are device pointers, so it
 // can be captured in a CUDA graph and replayed.

@@ -24,15 +24,17 @@
 //
 // B200 design: one cooperative persistent launch per solve.  Pull iterations
 // use the cached all-vertex sweep schedule (sweep.cuh): 32 consecutive
-// vertices per warp with a segmented shuffle reduction per owner vertex,
-// heavy vertices as tiles whose partial sums meet in an accumulator, a
-// contribution array c[u] = value[u]/nout[u] (SoA, double-buffered) so each
-// arc costs one 4-byte column read and one 4-byte gather, and the L1 change
-// reduced in fp64.  On a degree-ordered graph pull-topological runs over a
-// binned layout instead (pr_pull_binned, below).  Residual push (Sync) reuses the frontier queues
-// (frontier.cuh); Async runs over the device worklist (gb_worklist.cuh): a
-// warp keeps working on the vertices it activated itself, surplus goes to
-// the ring, and the launch ends when the worklist's work count reaches zero.
+// vertices per warp, eight lanes to a row (chunk_row_sums), heavy vertices as
+// tiles whose partial sums meet in an accumulator, a contribution array
+// c[u] = value[u]/nout[u] (SoA, double-buffered) so each arc costs one 4-byte
+// column read and one 4-byte gather, and the L1 change reduced in fp64.  In
+// file order the columns of a power-law graph are renamed by falling in-degree
+// (ensure_hot).  On a degree-ordered graph both pull variants run over a
+// binned layout instead (pr_pull_binned, below).  Residual push (Sync) reuses
+// the frontier queues (frontier.cuh); Async runs over the device worklist
+// (gb_worklist.cuh): a warp keeps working on the vertices it activated itself,
+// surplus goes to the ring, and the launch ends when the worklist's work count
+// reaches zero.
 
 #include <cub/cub.cuh>
 
@@ -276,12 +278,6 @@ __device__ __forceinline__ float tile_row_sum(const uint32_t* __restrict__ col, 
   return warp_sum(sum);
 }
 
-// Jacobi pull iterations, one cooperative persistent launch.  Shared memory
-// is kept small (one float per lane) so that the SM's unified L1/shared array
-// serves as L1 for the gathers; on a degree-ordered graph the hot
-// contributions sit on few lines and stay there.  On such a graph the
-// vertices from zero_from on have no in-arcs, so after two iterations their
-// rank and contribution are constants and their chunks are skipped.
 // Publish this thread's share of the iteration's L1 / max change: summed per
 // CTA in shared memory, then one atomic per CTA into one of kL1Slots words
 // (an atomic per warp on one word serialised ~7 K atomics per iteration), the
@@ -329,6 +325,12 @@ __device__ __forceinline__ void clear_change(PrCtl* ctl, uint32_t slot_set) {
   ctl->linf[slot_set] = 0u;
 }
 
+// Jacobi pull iterations, one cooperative persistent launch.  Shared memory
+// holds only the change's totals, so the SM's unified L1/shared array serves as
+// L1 for the gathers: the hot contributions sit on few lines (degree order, or
+// renamed columns) and stay there.  On a degree-ordered graph the vertices from
+// zero_from on have no in-arcs, so after two iterations their rank and
+// contribution are constants and their chunks are skipped.
 template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) pr_pull_persistent(PrArgs a) {
   __shared__ double s_l1, s_total;
