@@ -477,11 +477,11 @@ def _star_with_path(k, plen):
 @pytest.mark.parametrize("case", ["hub-split", "directed", "single-partition", "many-partitions"])
 def test_pagerank_binned_layout(cuda_device, case):
     """Degree-ordered graphs run PageRank pull and pull-residual over the
-    binned layout (partitions of 32 768 destinations, 256-arc chunks).
-    Shapes that exercise it: a hub whose partition is split over several
-    tasks (sums added with atomics), a directed graph with rows that have no
-    arcs but sources that do, a graph smaller than one partition, and one of
-    several partitions.  Pull against the FP64 Jacobi oracle (<= 1e-5,
+    binned layout (blocks of 32 768 sources, runs of arcs into one
+    destination, 256-arc chunks).  Shapes that exercise it: a hub whose run
+    spans whole chunks of several tasks and whose own block is split over
+    tasks, a directed graph with rows that have no arcs but sources that do, a
+    graph smaller than one block, and one of several blocks.  Pull against the FP64 Jacobi oracle (<= 1e-5,
     iterations within 2) and against the file-order row sweep (<= 1e-6);
     pull-residual against the FP64 restatement of its rounds
     (check_residual_parity, rounds within 2)."""
@@ -513,6 +513,28 @@ def test_pagerank_binned_layout(cuda_device, case):
         rgot, rst = dg.pagerank_pull_residual(0.85, 1e-4, 1000, stats=True)
         check_residual_parity(rgot, rwant, 1e-4, f"pull-residual {case}")
         assert abs(rst["iterations"] - rit) <= 2, case
+
+
+@pytest.mark.parametrize("heavy", [2, 4, 128])
+def test_pagerank_binned_more_heavy_rows_than_hubs(cuda_device, heavy):
+    """The binned layout adds the largest rows up in 64 bits, at most 16 384 of
+    them: with low degree thresholds a graph of 40 K vertices has more heavy
+    rows than that, with the default fewer.  Against the FP64 oracles as in
+    the layout's other test."""
+    g = erdos_renyi(40000, 9.0, seed=4)
+    assert (g.degrees() > 4).sum() > 16384 > (g.degrees() > 128).sum()
+    want, it64 = oracle.pr_pull_topo_f64(g, 0.85, 1e-6, 1000)
+    rwant, rit = oracle.pr_pull_residual(g, 0.85, 1e-4, 1000, f64=True)
+    with DeviceGraph(g, symmetric=True, reorder=_lib.GB_ORDER_DEGREE) as dg:
+        dg.set_tuning(heavy_degree=heavy)
+        for _ in range(2):
+            got, st = dg.pagerank_pull(0.85, 1e-6, 1000, stats=True)
+            assert np.max(np.abs(got.astype(np.float64) - want)) <= 1e-5
+            assert np.allclose(got, want, rtol=1e-4, atol=0)
+            assert abs(st["iterations"] - it64) <= 2
+        rgot, rst = dg.pagerank_pull_residual(0.85, 1e-4, 1000, stats=True)
+        check_residual_parity(rgot, rwant, 1e-4, f"pull-residual heavy={heavy}")
+        assert abs(rst["iterations"] - rit) <= 2
 
 
 @pytest.mark.parametrize("n", [4097, 20000])

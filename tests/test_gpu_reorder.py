@@ -250,12 +250,14 @@ def test_auto_order_and_default_region_kernel(cuda_device):
 @pytest.mark.parametrize("rows,cols,shift,region", [
     (1, 2047, 13, True), (1, 2048, 13, True), (33, 65, 13, True), (90, 433, 13, True), (601, 433, 13, True),
     (90, 433, 8, False), (90, 433, 14, False), (700, 120, 8, False), (700, 120, 11, True), (700, 120, 20, True),
-    (100, 2000, 13, False), (100, 2900, 13, False)])
+    (100, 2000, 13, False), (100, 2900, 13, False),
+    (20000, 16, 13, True), (1500, 250, 13, False)])
 @pytest.mark.parametrize("shuffled", [False, True])
 def test_default_region_rule_in_file_order(cuda_device, rows, cols, shift, region, shuffled):
     """A grid in file order takes the region kernel when its regions of 2048
     ids keep most of the arcs, no arc spans more ids than that and a bucket
-    holds enough hops, and not too many where the regions keep fewer; with the
+    holds enough hops, and not too many where the regions keep fewer or some
+    have no SM of their own (20 000 x 16: 157 regions that keep 99 %); with the
     ids shuffled only a graph of one region does.  Same distances either way,
     from the first vertex, the middle and the last."""
     g = grid2d(rows, cols)
