@@ -1589,7 +1589,7 @@ int run_pagerank(gb_graph* g, PrKind kind, float alpha, float tol, uint32_t max_
     // the flat sweep needs the degree order: heavy rows first, the light rows' arcs one range
     if (g->perm && (g->order == GB_ORDER_DEGREE || g->order == GB_ORDER_DEGREE_UNSORTED)) {
       // degree-ordered: the binned layout (sequential streams, few
-      // (source, partition) pairs per arc); where it cannot be built, the
+      // (block, destination) runs per arc); where it cannot be built, the
       // flat sweep (heavy rows are [0, nheavy), the light rows' arcs one
       // contiguous range)
       if (ensure_pr_bins(g, s) == GB_OK) {
